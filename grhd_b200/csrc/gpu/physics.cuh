@@ -672,8 +672,21 @@ __device__ inline double root_brent(double g1, double rho_floor, double D, doubl
   }
   return -1.0;
 }
-// equations.f90:249-340
-__device__ inline double root_safe_newton(double g1, double rho_floor, double D, double tau, double Q2, unsigned &flags) {
+// FP32 estimate of the residual and its derivative for E = tau + D scaled out:
+// f / E^2 and f' / E^2 at W, d = D / E, q = Q2 / E^2.  For g1 >= 1.9 and d <= 1.25 the factor V
+// is at most 2.1, so the error of f is below 1e-5 and that of f' below 1e-5 (1 + d W) / W^3.
+struct RootScreen {
+  float g1, d, q;
+  __device__ __forceinline__ void eval(float W, float &f, float &df) const {
+    const float W2 = W * W, iden = __fdividef(1.0f, g1 * W2 - 1.0f), iW = __fdividef(1.0f, W);
+    const float V = (g1 * W2 - d * W) * iden;
+    const float dV = (g1 * W * (d * W - 2.0f) + d) * (iden * iden);
+    f = V * V * (1.0f - iW * iW) - q;
+    df = 2.0f * V * (dV * (W2 * W - W) + V) * (iW * iW * iW);
+  }
+};
+// equations.f90:249-340, every residual in FP64
+__device__ inline double root_reference(double g1, double rho_floor, double D, double tau, double Q2, unsigned &flags) {
   const double x_acc = 1.0e-10, x1 = 1.0;
   double f_low, f_high, df, f, root, dx, dx_old, tmp;
   residual(g1, x1, D, tau, Q2, f_low, df);
@@ -710,6 +723,80 @@ __device__ inline double root_safe_newton(double g1, double rho_floor, double D,
   }
   flags |= C2P_BRENT;
   return root_brent(g1, rho_floor, D, tau, Q2);
+}
+// The FP64 path's rare branches out of line: its kernels carry one copy beside the common
+// path.  (The mixed root finder inlines root_reference: a call there costs its stage kernel
+// 3 % on 1024-cell grids.)
+static __device__ __noinline__ double root_reference_call(double g1, double rho_floor, double D, double tau, double Q2,
+                                                          unsigned &flags) {
+  return root_reference(g1, rho_floor, D, tau, Q2, flags);
+}
+static __device__ __noinline__ double root_brent_call(double g1, double rho_floor, double D, double tau, double Q2) {
+  return root_brent(g1, rho_floor, D, tau, Q2);
+}
+// The same root from fewer FP64 residuals.  The reference starts at the middle of
+// [1, max(1e3, 2 W_guess)] and bisects about ten times before Newton's step is accepted (12.4
+// residuals per torus cell, each four FP64 quotients).  A bisection's next iterate depends
+// on the residual only through two decisions -- bisect or Newton, and the sign of f -- so
+// while the FP32 estimate settles both with a margin (1e-4 E^2 against its error of 1e-5 E^2,
+// and an FP64 round-off of 1e-15 E^2), the bracket is halved in FP64 without evaluating the
+// residual in FP64.  From the first decision the estimate cannot settle on, the reference's
+// iteration continues unchanged: the iterates, and the root, are the same to the bit
+// (tests/test_gpu_root.py).  Measured with ncu on 8 tori 400x1x200, stage 1: FP64
+// instructions of the cell update 29.2e6 -> 17.9e6, 122 -> 111 us.
+__device__ inline double root_safe_newton(double g1, double rho_floor, double D, double tau, double Q2, unsigned &flags) {
+  const float Ef = (float)(tau + D), Df = (float)D, Qf = (float)Q2;
+  // V is finite at W = 1 for these operands, so f(1) = V^2 (1 - 1/1) - Q2 = -Q2
+  if (!(Ef > 1.0e-12f && Ef < 1.0e12f && Df > 0.0f && Df <= 1.25f * Ef && Qf < 1.0e24f && Q2 >= 0.0 && g1 >= 1.9))
+    return root_reference_call(g1, rho_floor, D, tau, Q2, flags);
+  if (Q2 < 1.0e-14) return 1.0;
+  const double x2 = rmax(1.0e3, (sqrt(Q2) + D) / rmax(D, rho_floor) * 2.0);
+  const float iE = __fdividef(1.0f, Ef);
+  const RootScreen scr{(float)g1, Df * iE, Qf * iE * iE};
+  float fs, dfs;
+  scr.eval((float)x2, fs, dfs);  // f(x2) certainly positive and not "zero": the bracket is [1, x2]
+  if (!((float)x2 < 1.0e5f && fs > 1.0e-4f && fs * Ef * Ef > 2.0e-14f))
+    return root_reference_call(g1, rho_floor, D, tau, Q2, flags);
+  double x_low = 1.0, x_high = x2, root = 0.5 * (1.0 + x2), dx = x2 - 1.0, dx_old = dx, f, df;
+  bool sign_open = false;  // the sign of f at root is not in the bracket yet
+  int it = 0;
+  {
+    float of = (float)dx_old, nf = of;  // dx_old, dx
+    scr.eval((float)root, fs, dfs);
+    while (nf > 1.0e-2f && fabsf(2.0f * fs) > 1.01f * fabsf(of * dfs) + 2.0e-4f) {  // bisection for certain
+      dx_old = dx;
+      dx = 0.5 * (x_high - x_low);
+      root = x_low + dx;
+      ++it;
+      of = nf;
+      nf = (float)dx;
+      scr.eval((float)root, fs, dfs);
+      sign_open = !(fabsf(fs) > 1.0e-4f);
+      if (sign_open) break;
+      if (fs < 0.0f) x_low = root; else x_high = root;
+    }
+  }
+  for (;; ++it) {
+    residual(g1, root, D, tau, Q2, f, df);
+    if (sign_open) { if (f < 0.0) x_low = root; else x_high = root; }
+    sign_open = true;
+    if (it == 100) break;
+    if (((root - x_high) * df - f) * ((root - x_low) * df - f) > 0.0 || fabs(2.0 * f) > fabs(dx_old * df)) {
+      dx_old = dx;
+      dx = 0.5 * (x_high - x_low);
+      root = x_low + dx;
+      if (fabs(x_low - root) < 1.0e-14) return root;
+    } else {
+      dx_old = dx;
+      dx = f / df;
+      const double tmp = root;
+      root = root - dx;
+      if (fabs(tmp - root) < 1.0e-14) return root;
+    }
+    if (fabs(dx) < 1.0e-10) return root;
+  }
+  flags |= C2P_BRENT;
+  return root_brent_call(g1, rho_floor, D, tau, Q2);
 }
 
 // Mixed-policy root finder: the residual and bracket [1, max(1e3, 2 W_guess)] of
@@ -750,7 +837,7 @@ __device__ inline double root_seeded_newton(double g1, double rho_floor, double 
     }
     root = next;
   }
-  return root_safe_newton(g1, rho_floor, D, tau, Q2, flags);
+  return root_reference(g1, rho_floor, D, tau, Q2, flags);
 }
 
 // cons_to_prim, equations.f90:94-205: cons modified in place (intent(inout)); returns flags.
