@@ -4,6 +4,8 @@
 // through shared-memory staging (k_cell_update).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace grhd {
@@ -122,14 +124,15 @@ __device__ __forceinline__ void c2p_count(unsigned long long *cnt, unsigned fl) 
 // MODE 0 writes the RHS only; MODE 1..3 are the SSP-RK3 stages (stage 1 also copies
 // up into u, the "u = up" of grhd2.f90:232).
 // ------------------------------------------------------------------------------------
-// Batched: block b works on grid map[b].grid, cell tile map[b].first / 128.
-// Resident 128-thread blocks per SM the register allocation must allow.  The kernel waits
-// on dependent FP64 chains (con2prim) and scattered table loads, so more warps in flight
-// pay for a few spilled registers: measured on the 2.5D and 3D torus batches, 8 blocks
-// (64 registers) is fastest for FP64 (6: -4 %, 4: -14 %) and 5 (96 registers, a third of
-// the spills of 6) for the mixed policy (6: -1 %, 4, 7 and 8 slower).
-template <class PT>
-constexpr int cell_min_blocks() { return sizeof(PT) == sizeof(double) ? 8 : 5; }
+// Batched: block b works on grid map[b].grid, cell tile map[b].first / block size.
+// Resident blocks per SM the register allocation must allow.  The kernel waits on dependent
+// FP64 chains (con2prim) and scattered table loads, so more warps in flight pay for a few
+// spilled registers: measured on the 2.5D and 3D torus batches, 1024 threads (64 registers)
+// is fastest for FP64 (896: -5 %, 768: -13 %, 1280: -5 % with 256-thread blocks) and 5 blocks
+// of 128 (96 registers, a third of the spills of 6) for the mixed policy (6: -1 %, 4, 7 and 8
+// slower).
+template <class PT, int LB>
+constexpr int cell_min_blocks() { return sizeof(PT) == sizeof(double) ? 1024 >> LB : 640 >> LB; }
 
 // cp.async (sm_80+ asynchronous global->shared copy, cp-size 4, 8 or 16 bytes) and its
 // commit/wait; a thread waits for its own groups only.
@@ -215,9 +218,9 @@ __device__ __forceinline__ void stage_slice(T *slice, const T *C, const GridDev 
   cp_async_commit();
 }
 
-// Where cell_core reads a cell's streamed inputs: the primitives, the two faces of each
-// active direction, and up, u.  DirectIn loads them from global memory where they are
-// used; StagedIn (below) has them copied into shared memory ahead of use.
+// Where cell_core reads a cell's streamed inputs (CellIn, below): the primitives, the two
+// faces of each active direction, and up, u, each either from global memory where it is used
+// or from shared memory, copied there ahead of use.
 struct CellIndex {
   long long c;     // cell index in the state planes
   unsigned i, j, k;
@@ -240,23 +243,105 @@ __device__ __forceinline__ long long face_up(const GridDev &G, int d) {
   return d == 0 ? 1LL : (d == 1 ? (long long)G.nx : (long long)G.nx * G.ny);
 }
 
-template <class R, class PT, class ColR = GlobalCol<R>, class Col64 = GlobalCol<double>>
-struct DirectIn {
-  const GridDev &G;
-  const CellIndex &x;
+// ---- staged inputs ------------------------------------------------------------------
+// The inputs of the mask ST (STAGE_P primitives, STAGE_F face fluxes, STAGE_U up and u) are
+// copied by each thread for its own cell into shared memory with cp.async (sm_80+
+// asynchronous global->shared copies; a thread waits for its own groups, so no block barrier
+// is needed), one commit group each: all the copies are in flight at once without holding
+// registers, and the sources (which need only the primitives and the metric tables) overlap
+// the flux and RK-state fetches.  Layout per block of BS threads, structure of arrays:
+//   double up[NEQ][BS], u[NEQ][BS]; PT p[NEQ][BS];
+//   R f[2 * dirs][NEQ][BS]   (lower, upper face of each active direction)
+constexpr int STAGE_P = 1, STAGE_F = 2, STAGE_U = 4, STAGE_ALL = 7;
+__host__ __device__ constexpr int stage_groups(int st) { return ((st & 1) != 0) + ((st & 2) != 0) + ((st & 4) != 0); }
+template <class R, class PT, int ST, int BS>
+__host__ __device__ constexpr size_t cell_stage_bytes(int dirs) {
+  return (size_t)BS * NEQ *
+         (((ST & STAGE_U) ? 2 * sizeof(double) : 0) + ((ST & STAGE_P) ? sizeof(PT) : 0) + ((ST & STAGE_F) ? 2 * dirs * sizeof(R) : 0));
+}
+
+template <class R, class PT, int ST, int BS, class ColR = GlobalCol<R>, class Col64 = GlobalCol<double>>
+struct CellIn {
+  const GridDev *G;
+  CellIndex x;
   ColR cr;     // the centre table of arithmetic type R (sources)
   Col64 c64;   // the FP64 centre table (con2prim metric)
-  __device__ __forceinline__ void wait_prims() const {}
-  __device__ __forceinline__ void wait_fluxes() const {}
-  __device__ __forceinline__ void wait_state() const {}
+  const double *s_up, *s_u;
+  const PT *s_p;
+  const R *s_f;
+  int t, slot[3];
+  __device__ __forceinline__ CellIn(const GridDev &G_, const CellIndex &x_, ColR cr_, Col64 c64_)
+      : G(&G_), x(x_), cr(cr_), c64(c64_) {}
   __device__ __forceinline__ const ColR &table_r() const { return cr; }
   __device__ __forceinline__ const Col64 &table64() const { return c64; }
-  __device__ __forceinline__ double prim(int v) const { return (double)((const PT *)G.P)[v * G.pplane + x.c]; }
-  __device__ __forceinline__ R flux(int d, int upper, int v) const {
-    return ((const R *)G.F[d])[v * face_n(G, d) + face_lo(G, x, d) + (upper ? face_up(G, d) : 0)];
+  // issue the copy groups of this thread's cell: primitives, face fluxes, up and u
+  __device__ __forceinline__ void issue(const int MODE, unsigned char *raw) {
+    t = threadIdx.x;
+    double *up = (double *)raw;
+    double *u = up + ((ST & STAGE_U) ? NEQ * BS : 0);
+    PT *p = (PT *)(u + ((ST & STAGE_U) ? NEQ * BS : 0));
+    R *f = (R *)(p + ((ST & STAGE_P) ? NEQ * BS : 0));
+    s_up = up; s_u = u; s_p = p; s_f = f;
+    slot[0] = 0;
+    slot[1] = 1;
+    slot[2] = G->ny > 1 ? 2 : 1;
+    if constexpr ((ST & STAGE_P) != 0) {
+      const PT *Pg = (const PT *)G->P;
+#pragma unroll
+      for (int v = 0; v < NEQ; ++v) cp_async<sizeof(PT)>(&p[v * BS + t], &Pg[v * G->pplane + x.c]);
+      cp_async_commit();
+    }
+    if constexpr ((ST & STAGE_F) != 0) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        if ((d == 1 && G->ny == 1) || (d == 2 && G->nz == 1)) continue;
+        const R *Fg = (const R *)G->F[d];
+        const long long lo = face_lo(*G, x, d), nf = face_n(*G, d), off = face_up(*G, d);
+#pragma unroll
+        for (int v = 0; v < NEQ; ++v) {
+          cp_async<sizeof(R)>(&f[((2 * slot[d]) * NEQ + v) * BS + t], &Fg[v * nf + lo]);
+          cp_async<sizeof(R)>(&f[((2 * slot[d] + 1) * NEQ + v) * BS + t], &Fg[v * nf + lo + off]);
+        }
+      }
+      cp_async_commit();
+    }
+    if constexpr ((ST & STAGE_U) != 0) {
+      if (MODE != 0) {
+#pragma unroll
+        for (int v = 0; v < NEQ; ++v) cp_async<8>(&up[v * BS + t], &G->UP[v * G->pplane + x.c]);
+        if (MODE >= 2) {
+#pragma unroll
+          for (int v = 0; v < NEQ; ++v) cp_async<8>(&u[v * BS + t], &G->U[v * G->pplane + x.c]);
+        }
+      }
+      cp_async_commit();
+    }
   }
-  __device__ __forceinline__ double up(int v) const { return G.UP[v * G.pplane + x.c]; }
-  __device__ __forceinline__ double u(int v) const { return G.U[v * G.pplane + x.c]; }
+  __device__ __forceinline__ void wait_prims() const {
+    if constexpr ((ST & STAGE_P) != 0) cp_async_wait<stage_groups(ST & (STAGE_F | STAGE_U))>();
+  }
+  __device__ __forceinline__ void wait_fluxes() const {
+    if constexpr ((ST & STAGE_F) != 0) cp_async_wait<stage_groups(ST & STAGE_U)>();
+  }
+  __device__ __forceinline__ void wait_state() const {
+    if constexpr ((ST & STAGE_U) != 0) cp_async_wait<0>();
+  }
+  __device__ __forceinline__ double prim(int v) const {
+    if constexpr ((ST & STAGE_P) != 0) return (double)s_p[v * BS + t];
+    else return (double)((const PT *)G->P)[v * G->pplane + x.c];
+  }
+  __device__ __forceinline__ R flux(int d, int upper, int v) const {
+    if constexpr ((ST & STAGE_F) != 0) return s_f[((2 * slot[d] + upper) * NEQ + v) * BS + t];
+    else return ((const R *)G->F[d])[v * face_n(*G, d) + face_lo(*G, x, d) + (upper ? face_up(*G, d) : 0)];
+  }
+  __device__ __forceinline__ double up(int v) const {
+    if constexpr ((ST & STAGE_U) != 0) return s_up[v * BS + t];
+    else return G->UP[v * G->pplane + x.c];
+  }
+  __device__ __forceinline__ double u(int v) const {
+    if constexpr ((ST & STAGE_U) != 0) return s_u[v * BS + t];
+    else return G->U[v * G->pplane + x.c];
+  }
 };
 
 // Seed of the mixed policy's root finder: the Lorentz factor of the cell's primitives at
@@ -450,103 +535,34 @@ __device__ __forceinline__ void cell_item(const GridDev &G, unsigned ia, unsigne
   const CellIndex x = cell_index_of(G, ia, jb, kc);
   const long long ij = (long long)ia + (long long)G.nx * jb;
   cell_core<R, PT>(G, ia, jb, x, MODE, dt,
-                   DirectIn<R, PT>{G, x, global_col(centre_table<R>(G), G, ij), global_col(G.centre, G, ij)});
+                   CellIn<R, PT, 0, 1>(G, x, global_col(centre_table<R>(G), G, ij), global_col(G.centre, G, ij)));
 }
 
-// ---- staged inputs ------------------------------------------------------------------
-// Each thread copies its own cell's streamed inputs into shared memory with cp.async
-// (sm_80+ asynchronous global->shared copies; a thread waits for its own groups, so no
-// block barrier is needed) in three commit groups: primitives, face fluxes, then up and
-// u.  All the copies are in flight at once without holding registers, and the sources
-// (which need only the primitives and the metric tables) overlap the flux and RK-state
-// fetches.  Layout per block, structure of arrays over the block's threads:
-//   double up[NEQ][CELL_BS], u[NEQ][CELL_BS]; PT p[NEQ][CELL_BS];
-//   R f[2 * dirs][NEQ][CELL_BS]   (lower, upper face of each active direction)
-constexpr int CELL_BS_STAGE = 128;
-static_assert(CELL_BS_STAGE % 32 == 0, "sliced cell tiles are whole warps along i");
-// Staging pays for the mixed policy (measured on the 2.5D and 3D torus batches: cell
-// update -7 %); the FP64 kernel is bound by its FP64 instruction stream and runs as fast
-// with direct loads and no shared memory limiting its resident blocks.
-template <class PT>
-__host__ __device__ constexpr bool cell_staged() { return sizeof(PT) == sizeof(float); }
-template <class R, class PT>
-__host__ __device__ constexpr size_t cell_stage_bytes(int dirs) {
-  return cell_staged<PT>()
-             ? (size_t)CELL_BS_STAGE * (2 * NEQ * sizeof(double) + NEQ * sizeof(PT) + 2 * dirs * NEQ * sizeof(R))
-             : 0;
+constexpr int CELL_LB = 7, CELL_LB_WIDE = 8;  // log2 of the block sizes (flux_launch.h CELL_BS, CELL_BS_WIDE)
+// What a kernel stages.  Mixed policy: everything (cell update -7 %).  FP64: 128-thread blocks
+// load directly; 256-thread blocks stage up and u, whose loads come last and wait longest.
+template <class PT, int LB>
+__host__ __device__ constexpr int cell_stage_mask() {
+  return sizeof(PT) == sizeof(float) ? STAGE_ALL : (LB == CELL_LB_WIDE ? STAGE_U : 0);
 }
 
-template <class R, class PT, class ColR, class Col64>
-struct StagedIn {
-  const double *s_up, *s_u;
-  const PT *s_p;
-  const R *s_f;
-  int t, slot[3];
-  ColR cr;
-  Col64 c64;
-  __device__ __forceinline__ StagedIn(ColR cr_, Col64 c64_) : cr(cr_), c64(c64_) {}
-  __device__ __forceinline__ const ColR &table_r() const { return cr; }
-  __device__ __forceinline__ const Col64 &table64() const { return c64; }
-  // issue the three copy groups (primitives, face fluxes, up and u) of this thread's cell
-  __device__ __forceinline__ void issue(const GridDev &G, const CellIndex &x, const int MODE, unsigned char *raw) {
-    t = threadIdx.x;
-    double *up = (double *)raw;
-    double *u = up + NEQ * CELL_BS_STAGE;
-    PT *p = (PT *)(u + NEQ * CELL_BS_STAGE);
-    R *f = (R *)(p + NEQ * CELL_BS_STAGE);
-    s_up = up; s_u = u; s_p = p; s_f = f;
-    slot[0] = 0;
-    slot[1] = 1;
-    slot[2] = G.ny > 1 ? 2 : 1;
-    const PT *Pg = (const PT *)G.P;
-#pragma unroll
-    for (int v = 0; v < NEQ; ++v) cp_async<sizeof(PT)>(&p[v * CELL_BS_STAGE + t], &Pg[v * G.pplane + x.c]);
-    cp_async_commit();
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      if ((d == 1 && G.ny == 1) || (d == 2 && G.nz == 1)) continue;
-      const R *Fg = (const R *)G.F[d];
-      const long long lo = face_lo(G, x, d), nf = face_n(G, d), off = face_up(G, d);
-#pragma unroll
-      for (int v = 0; v < NEQ; ++v) {
-        cp_async<sizeof(R)>(&f[((2 * slot[d]) * NEQ + v) * CELL_BS_STAGE + t], &Fg[v * nf + lo]);
-        cp_async<sizeof(R)>(&f[((2 * slot[d] + 1) * NEQ + v) * CELL_BS_STAGE + t], &Fg[v * nf + lo + off]);
-      }
-    }
-    cp_async_commit();
-    if (MODE != 0) {
-#pragma unroll
-      for (int v = 0; v < NEQ; ++v) cp_async<8>(&up[v * CELL_BS_STAGE + t], &G.UP[v * G.pplane + x.c]);
-      if (MODE >= 2) {
-#pragma unroll
-        for (int v = 0; v < NEQ; ++v) cp_async<8>(&u[v * CELL_BS_STAGE + t], &G.U[v * G.pplane + x.c]);
-      }
-    }
-    cp_async_commit();
-  }
-  __device__ __forceinline__ void wait_prims() const { cp_async_wait<2>(); }
-  __device__ __forceinline__ void wait_fluxes() const { cp_async_wait<1>(); }
-  __device__ __forceinline__ void wait_state() const { cp_async_wait<0>(); }
-  __device__ __forceinline__ double prim(int v) const { return (double)s_p[v * CELL_BS_STAGE + t]; }
-  __device__ __forceinline__ R flux(int d, int upper, int v) const {
-    return s_f[((2 * slot[d] + upper) * NEQ + v) * CELL_BS_STAGE + t];
-  }
-  __device__ __forceinline__ double up(int v) const { return s_up[v * CELL_BS_STAGE + t]; }
-  __device__ __forceinline__ double u(int v) const { return s_u[v * CELL_BS_STAGE + t]; }
-};
-
-// Dynamic shared memory: the table slice (slice_bytes<R>()), then for the mixed policy the
-// staged inputs (cell_stage_bytes<R, PT>(dirs); dirs = the most active directions of any
-// grid of the launch).
-template <int MODE, class R, class PT>
-__global__ void __launch_bounds__(CELL_BS_STAGE, cell_min_blocks<PT>())
+// Dynamic shared memory: the table slice (slice_bytes<R>()), then the staged inputs
+// (cell_stage_bytes; dirs = the most active directions of any grid of the launch).
+template <class R, class PT, int LB>
+__host__ __device__ constexpr size_t cell_smem_bytes(int dirs) {
+  return slice_bytes<R>() + cell_stage_bytes<R, PT, cell_stage_mask<PT, LB>(), 1 << LB>(dirs);
+}
+template <int MODE, class R, class PT, int LB>
+__global__ void __launch_bounds__(1 << LB, cell_min_blocks<PT, LB>())
     k_cell_update(const GridDev *__restrict__ grids, const BlockMap *__restrict__ map) {
   extern __shared__ __align__(16) unsigned char cell_stage[];
+  constexpr int ST = cell_stage_mask<PT, LB>(), BS = 1 << LB;
+  static_assert(BS % 32 == 0, "sliced cell tiles are whole warps along i");
   const BlockMap bm = map[blockIdx.x];
   const GridDev &G = grids[bm.grid];
   unsigned ia, jb, kc;
-  const bool valid = tile_item<7>(G.tiles[TILE_CELL], (unsigned)bm.first >> 7, threadIdx.x, (unsigned)G.nx,
-                                  (unsigned)G.ny, (unsigned)G.nz, ia, jb, kc);
+  const bool valid = tile_item<LB>(G.tiles[TILE_CELL], (unsigned)bm.first >> LB, threadIdx.x, (unsigned)G.nx,
+                                   (unsigned)G.ny, (unsigned)G.nz, ia, jb, kc);
   double dt = 0.0;
   if (MODE != 0) {
     const GridClock ck = *G.clock;
@@ -556,31 +572,21 @@ __global__ void __launch_bounds__(CELL_BS_STAGE, cell_min_blocks<PT>())
   const unsigned lane = threadIdx.x & 31u;
   const bool sliced = cell_tile_sliced(G);  // the same for the whole block
   R *slice = (R *)cell_stage;
+  unsigned char *inputs = cell_stage + slice_bytes<R>();
   if (sliced) stage_slice<R>(slice, centre_table<R>(G), G, ia - lane, jb);
   const CellIndex x = cell_index_of(G, ia, jb, kc);
   const long long ij = (long long)ia + (long long)G.nx * jb;
-  if (!cell_staged<PT>()) {  // FP64: direct loads of the streamed inputs
-    if (sliced) {
-      cp_async_wait<0>();
-      __syncthreads();
-    }
-    if (!valid) return;
-    if (sliced)
-      cell_core<R, PT>(G, ia, jb, x, MODE, dt,
-                       DirectIn<R, PT, SliceCol<R>, SliceCol<R>>{G, x, SliceCol<R>{slice, lane}, SliceCol<R>{slice, lane}});
-    else
-      cell_core<R, PT>(G, ia, jb, x, MODE, dt,
-                       DirectIn<R, PT>{G, x, global_col(centre_table<R>(G), G, ij), global_col(G.centre, G, ij)});
-    return;
-  }
-  // mixed policy: the FP32 table from the slice, the FP64 metric of con2prim from global
-  // memory field by field
-  unsigned char *inputs = cell_stage + slice_bytes<R>();
+  // con2prim's FP64 metric: the slice itself in FP64, from global memory field by field in
+  // the mixed policy
   if (sliced) {
-    StagedIn<R, PT, SliceCol<R>, LazyCol<double>> in(SliceCol<R>{slice, lane}, LazyCol<double>{global_col(G.centre, G, ij)});
+    using C64 = std::conditional_t<sizeof(R) == sizeof(double), SliceCol<double>, LazyCol<double>>;
+    C64 c64;
+    if constexpr (sizeof(R) == sizeof(double)) c64 = SliceCol<double>{slice, lane};
+    else c64 = LazyCol<double>{global_col(G.centre, G, ij)};
+    CellIn<R, PT, ST, BS, SliceCol<R>, C64> in(G, x, SliceCol<R>{slice, lane}, c64);
     if (valid) {
-      in.issue(G, x, MODE, inputs);
-      cp_async_wait<3>();  // the slice's group; the three input groups stay in flight
+      in.issue(MODE, inputs);
+      cp_async_wait<stage_groups(ST)>();  // the slice's group; the input groups stay in flight
     } else {
       cp_async_wait<0>();
     }
@@ -589,9 +595,9 @@ __global__ void __launch_bounds__(CELL_BS_STAGE, cell_min_blocks<PT>())
     cell_core<R, PT>(G, ia, jb, x, MODE, dt, in);
   } else {
     if (!valid) return;
-    StagedIn<R, PT, GlobalCol<R>, LazyCol<double>> in(global_col(centre_table<R>(G), G, ij),
-                                                       LazyCol<double>{global_col(G.centre, G, ij)});
-    in.issue(G, x, MODE, inputs);
+    using C64 = std::conditional_t<sizeof(R) == sizeof(double), GlobalCol<double>, LazyCol<double>>;
+    CellIn<R, PT, ST, BS, GlobalCol<R>, C64> in(G, x, global_col(centre_table<R>(G), G, ij), C64{global_col(G.centre, G, ij)});
+    in.issue(MODE, inputs);
     cell_core<R, PT>(G, ia, jb, x, MODE, dt, in);
   }
 }

@@ -8,20 +8,31 @@
 
 namespace grhd {
 
-static_assert(CELL_BS == CELL_BS_STAGE, "the cell kernel's staging layout is per block thread");
+static_assert(CELL_BS == 1 << CELL_LB && CELL_BS_WIDE == 1 << CELL_LB_WIDE, "block sizes are the kernel's");
 
-// dirs: the most active directions of any grid in the launch (sizes the staging buffers)
-template <class R, class PT>
-void launch_cell(int mode, const GridDev *grids, const BlockMap *map, int nblocks, int dirs, cudaStream_t s) {
-  if (nblocks <= 0) return;
-  const unsigned nb = (unsigned)nblocks;
-  const size_t smem = slice_bytes<R>() + cell_stage_bytes<R, PT>(dirs);
+template <int LB, class R, class PT>
+inline void launch_cell_lb(int mode, const GridDev *grids, const BlockMap *map, unsigned nb, int dirs, cudaStream_t s) {
+  constexpr int bs = 1 << LB;
+  const size_t smem = cell_smem_bytes<R, PT, LB>(dirs);
   switch (mode) {
-    case 0: k_cell_update<0, R, PT><<<nb, CELL_BS, smem, s>>>(grids, map); break;
-    case 1: k_cell_update<1, R, PT><<<nb, CELL_BS, smem, s>>>(grids, map); break;
-    case 2: k_cell_update<2, R, PT><<<nb, CELL_BS, smem, s>>>(grids, map); break;
-    default: k_cell_update<3, R, PT><<<nb, CELL_BS, smem, s>>>(grids, map); break;
+    case 0: k_cell_update<0, R, PT, LB><<<nb, bs, smem, s>>>(grids, map); break;
+    case 1: k_cell_update<1, R, PT, LB><<<nb, bs, smem, s>>>(grids, map); break;
+    case 2: k_cell_update<2, R, PT, LB><<<nb, bs, smem, s>>>(grids, map); break;
+    default: k_cell_update<3, R, PT, LB><<<nb, bs, smem, s>>>(grids, map); break;
   }
+}
+// dirs: the most active directions of any grid in the launch (sizes the staging buffers);
+// wide: 256-thread blocks (FP64 only)
+template <class R, class PT>
+void launch_cell(int mode, bool wide, const GridDev *grids, const BlockMap *map, int nblocks, int dirs, cudaStream_t s) {
+  if (nblocks <= 0) return;
+  if constexpr (sizeof(PT) == sizeof(double)) {
+    if (wide) {
+      launch_cell_lb<CELL_LB_WIDE, R, PT>(mode, grids, map, (unsigned)nblocks, dirs, s);
+      return;
+    }
+  }
+  launch_cell_lb<CELL_LB, R, PT>(mode, grids, map, (unsigned)nblocks, dirs, s);
 }
 
 }  // namespace grhd

@@ -13,6 +13,7 @@ struct BlockMap;
 constexpr int RECON_BS = 256;
 constexpr int RIEMANN_BS = 128;
 constexpr int CELL_BS = 128;
+constexpr int CELL_BS_WIDE = 256;
 constexpr int FUSED_FLUX_BS = 128;  // k_flux (flux.cuh FLUX_BS)
 
 template <class R, class PT>
@@ -35,9 +36,9 @@ GRHD_FLUX_EXTERN(3, float, float)
 
 // stage cell kernel (cell_fp64.cu / cell_fp32.cu): mode 0 RHS only, 1..3 RK stages
 template <class R, class PT>
-void launch_cell(int mode, const GridDev *grids, const BlockMap *map, int nblocks, int dirs, cudaStream_t s);
-extern template void launch_cell<double, double>(int, const GridDev *, const BlockMap *, int, int, cudaStream_t);
-extern template void launch_cell<float, float>(int, const GridDev *, const BlockMap *, int, int, cudaStream_t);
+void launch_cell(int mode, bool wide, const GridDev *grids, const BlockMap *map, int nblocks, int dirs, cudaStream_t s);
+extern template void launch_cell<double, double>(int, bool, const GridDev *, const BlockMap *, int, int, cudaStream_t);
+extern template void launch_cell<float, float>(int, bool, const GridDev *, const BlockMap *, int, int, cudaStream_t);
 
 // stage kernel (stage.cuh): one whole RK stage (mode 1..3) of 1D grids (sd 0), x-y grids
 // (sd 2) or x-z grids (sd 3); tiles of STAGE_TILE_CELLS cells (256 along i, or 32 x 8),

@@ -50,12 +50,12 @@ int vfail(std::string &err, int code, const char *fmt, va_list ap) {
 // kernel kinds of a step and their items-per-block
 enum Kind {
   K_RECON_X = 0, K_RIEMANN_X, K_RECON_Y, K_RIEMANN_Y, K_RECON_Z, K_RIEMANN_Z, K_CELL, K_FLUX_X, K_FLUX_Y, K_FLUX_Z,
-  K_STAGE, NKIND
+  K_STAGE, K_CELL_WIDE, NKIND
 };
 const int KIND_BS[NKIND] = {RECON_BS, RIEMANN_BS, RECON_BS, RIEMANN_BS, RECON_BS, RIEMANN_BS, CELL_BS,
-                            FUSED_FLUX_BS, FUSED_FLUX_BS, FUSED_FLUX_BS, STAGE_BLOCK};
+                            FUSED_FLUX_BS, FUSED_FLUX_BS, FUSED_FLUX_BS, STAGE_BLOCK, CELL_BS_WIDE};
 const char *KIND_NAME[NKIND] = {"recon_x", "riemann_x", "recon_y", "riemann_y", "recon_z", "riemann_z",
-                                "cell_update", "flux_x", "flux_y", "flux_z", "stage"};
+                                "cell_update", "flux_x", "flux_y", "flux_z", "stage", "cell_update"};
 
 // ---- block tiles ------------------------------------------------------------------------
 unsigned ilog2(unsigned x) {
@@ -82,7 +82,7 @@ long long tile_count(const Tile &T, unsigned lb, unsigned nK) {
   const unsigned lz = lb - T.lx - T.ly;
   return (long long)T.nti.d * T.ntj.d * ((nK + (1u << lz) - 1) >> lz);
 }
-constexpr unsigned LB_RECON = 8, LB_FACE = 7, LB_CELL = 7;  // log2 of RECON_BS, RIEMANN_BS = FUSED_FLUX_BS, CELL_BS
+constexpr unsigned LB_CELL = CELL_LB, LB_RECON = 8, LB_FACE = 7;  // log2 of RECON_BS, RIEMANN_BS = FUSED_FLUX_BS, CELL_BS
 static_assert((1 << LB_RECON) == RECON_BS && (1 << LB_FACE) == RIEMANN_BS && (1 << LB_FACE) == FUSED_FLUX_BS &&
                   (1 << LB_CELL) == CELL_BS, "block sizes are the tile sizes");
 constexpr unsigned DEFAULT_TX = 32;
@@ -120,8 +120,10 @@ long long stage_tiles(const GridDev &G) {
 // threads (tiles x block size) a kernel kind launches for one grid
 long long kind_items(const GridDev &G, int k) {
   if (k == K_CELL) return tile_count(G.tiles[TILE_CELL], LB_CELL, (unsigned)G.nz) * CELL_BS;
+  // wide blocks keep the tile's 32 cells along i and take 8 along k
+  if (k == K_CELL_WIDE) return G.nz > 1 ? tile_count(G.tiles[TILE_CELL], LB_CELL + 1, (unsigned)G.nz) * CELL_BS_WIDE : 0;
   if (k == K_STAGE) return stage_tiles(G) * STAGE_BLOCK;
-  const int dir = k >= K_FLUX_X ? k - K_FLUX_X + 1 : k / 2 + 1;
+  const int dir = k >= K_FLUX_X && k <= K_FLUX_Z ? k - K_FLUX_X + 1 : k / 2 + 1;
   if (!dir_active(G, dir)) return 0;
   unsigned nI, nJ, nK;
   space_of(G, dir, nI, nJ, nK);
@@ -183,6 +185,7 @@ struct Group {
   int max_blocks = 0;  // resident blocks of the group's persistent instantiation
   int max_blocks_stage = 0;  // resident blocks of its persistent stage kernel (stage groups of 1D grids)
   int cell_dirs = 1;   // the most active directions of a member grid (cell kernel staging)
+  bool cell_wide = false;  // FP64 cell update in 256-thread blocks
   bool stage = false;  // steps run the stage kernel (one launch per stage) instead of face and cell kernels
 };
 
@@ -383,6 +386,21 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
   return b->stage_request == GRHD2_STAGE_ON || grp.sd == 0;
 }
 
+// Whether a group's FP64 cell update runs in 256-thread blocks (cell.cuh): eight warps share
+// a table slice instead of four, which leaves L1 75 KB more and shared memory room to stage
+// up and u.  Measured on k tori of 400x1x200 (325 wide blocks each), us per stage, narrow and
+// wide: k = 1 25.2 and 27.4, k = 2 38.0 and 36.2, k = 4 62.8 and 59.1, k = 12 157 and 146,
+// k = 32 405 and 376; 3D torus 256x128x128 635 and 568.  So wide blocks pay once they fill the
+// GPU (148 SMs x 4 resident blocks) more than once; below that the coarser blocks leave SMs
+// idle.  Every grid needs a k extent (other tiles share no slice).
+constexpr int WIDE_CELLS_FROM_BLOCKS = 148 * 4;
+bool use_wide_cells(const Group &grp, const std::vector<GridDev> &hg) {
+  if (grp.mixed || grp.nb[K_CELL_WIDE] < WIDE_CELLS_FROM_BLOCKS) return false;
+  for (int g : grp.members)
+    if (hg[g].nz == 1) return false;
+  return true;
+}
+
 // A scheme group of at least SPLIT_GROUP_CELLS cells over two or more grids runs as two
 // groups of about half the cells each, which a captured step runs as parallel branches of
 // its graph: each half's interface states stay closer to L2 and one half's kernel tails
@@ -465,6 +483,7 @@ int build_batch(grhd2_gpu_batch *b) {
       }
       grp.nb[k] = (int)map.size() - grp.off[k];
     }
+    grp.cell_wide = use_wide_cells(grp, hg);
     BCUDA_TRY(b, cudaMallocAsync((void **)&grp.d_map, sizeof(BlockMap) * std::max<size_t>(1, map.size()), b->stream));
     BCUDA_TRY(b, cudaMemcpyAsync(grp.d_map, map.data(), sizeof(BlockMap) * map.size(), cudaMemcpyHostToDevice, b->stream));
     // persistent kernel: flattened item spaces (faces of every active direction; cells)
@@ -549,8 +568,9 @@ int enqueue_fluxes(grhd2_gpu_batch *b, const Group &grp, cudaStream_t st) {
 
 template <int MODE, class R, class PT>
 int enqueue_cells(grhd2_gpu_batch *b, const Group &grp, cudaStream_t st) {
-  if (grp.nb[K_CELL] <= 0) return 0;
-  launch_cell<R, PT>(MODE, b->d_grids, grp.d_map + grp.off[K_CELL], grp.nb[K_CELL], grp.cell_dirs, st);
+  const int k = grp.cell_wide ? K_CELL_WIDE : K_CELL;
+  if (grp.nb[k] <= 0) return 0;
+  launch_cell<R, PT>(MODE, grp.cell_wide, b->d_grids, grp.d_map + grp.off[k], grp.nb[k], grp.cell_dirs, st);
   return blaunch_check(b, MODE == 0 ? "cell_rhs" : "cell_update");
 }
 

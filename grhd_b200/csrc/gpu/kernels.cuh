@@ -56,12 +56,12 @@ __global__ void k_c2p_all(const GridDev G, const Phys P, PT *__restrict__ Pout, 
 // the latency of its torus cells' ~30 residual evaluations; launched together, the grids'
 // waves overlap instead of running one after another.
 template <class PT>
-__global__ void __launch_bounds__(CELL_BS_STAGE, 8)
+__global__ void __launch_bounds__(1 << CELL_LB, 8)
     k_c2p_batch(const GridDev *__restrict__ grids, const BlockMap *__restrict__ map) {
   const BlockMap bm = map[blockIdx.x];
   const GridDev &G = grids[bm.grid];
   unsigned ia, jb, kc;
-  if (!tile_item<7>(G.tiles[TILE_CELL], (unsigned)bm.first >> 7, threadIdx.x, (unsigned)G.nx, (unsigned)G.ny,
+  if (!tile_item<CELL_LB>(G.tiles[TILE_CELL], (unsigned)bm.first >> CELL_LB, threadIdx.x, (unsigned)G.nx, (unsigned)G.ny,
                     (unsigned)G.nz, ia, jb, kc))
     return;
   const CellIndex x = cell_index_of(G, ia, jb, kc);
