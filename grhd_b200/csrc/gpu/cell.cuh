@@ -399,35 +399,38 @@ __device__ __forceinline__ void store_carry(const GridDev &G, void *C, long long
 // rounding error, up + rhs*dt, then u = up (stage 1), 0.75 u + 0.25 (...) (stage 2) or
 // (u + 2 (...)) / 3 (stage 3).  hi goes to con2prim as the stage's FP64 state, lo to the
 // carry.
+// One variable, at plane index k.
+__device__ __forceinline__ void rk_compensated(const GridDev &G, long long k, int MODE, double dt, double up, double u,
+                                               double rhs, double &hi, double &lo) {
+  const double upl = load_carry(G, G.UPc, k);
+  const double d = rhs * dt, dl = fma(rhs, dt, -d);
+  double th, tl;
+  dd_add(up, upl, d, dl, th, tl);  // up + rhs*dt
+  if (MODE == 1) {
+    G.U[k] = up;  // u = up (grhd2.f90:232), carry included
+    store_carry(G, G.Uc, k, upl);
+    hi = th;
+    lo = tl;
+  } else if (MODE == 2) {
+    double ah, al, bh, bl;
+    dd_mul(u, load_carry(G, G.Uc, k), 0.75, ah, al);
+    dd_mul(th, tl, 0.25, bh, bl);
+    dd_add(ah, al, bh, bl, hi, lo);
+  } else {
+    double sh, sl;
+    dd_add(u, load_carry(G, G.Uc, k), 2.0 * th, 2.0 * tl, sh, sl);
+    const double q = sh / 3.0;
+    const double ql = (fma(-q, 3.0, sh) + sl) / 3.0;
+    hi = q + ql;
+    lo = ql - (hi - q);
+  }
+}
 template <class In>
 __device__ __forceinline__ void rk_stage_compensated(const GridDev &G, long long c, int MODE, double dt, const In &in,
                                                      const double (&rhs)[NEQ], double (&hi)[NEQ], double (&lo)[NEQ]) {
 #pragma unroll
-  for (int v = 0; v < NEQ; ++v) {
-    const long long k = v * G.pplane + c;
-    const double up = in.up(v), upl = load_carry(G, G.UPc, k);
-    const double d = rhs[v] * dt, dl = fma(rhs[v], dt, -d);
-    double th, tl;
-    dd_add(up, upl, d, dl, th, tl);  // up + rhs*dt
-    if (MODE == 1) {
-      G.U[k] = up;  // u = up (grhd2.f90:232), carry included
-      store_carry(G, G.Uc, k, upl);
-      hi[v] = th;
-      lo[v] = tl;
-    } else if (MODE == 2) {
-      double ah, al, bh, bl;
-      dd_mul(in.u(v), load_carry(G, G.Uc, k), 0.75, ah, al);
-      dd_mul(th, tl, 0.25, bh, bl);
-      dd_add(ah, al, bh, bl, hi[v], lo[v]);
-    } else {
-      double sh, sl;
-      dd_add(in.u(v), load_carry(G, G.Uc, k), 2.0 * th, 2.0 * tl, sh, sl);
-      const double q = sh / 3.0;
-      const double ql = (fma(-q, 3.0, sh) + sl) / 3.0;
-      hi[v] = q + ql;
-      lo[v] = ql - (hi[v] - q);
-    }
-  }
+  for (int v = 0; v < NEQ; ++v)
+    rk_compensated(G, v * G.pplane + c, MODE, dt, in.up(v), MODE >= 2 ? in.u(v) : 0.0, rhs[v], hi[v], lo[v]);
 }
 
 // The new primitives go to Pout (the stage kernel's next buffer), or to G.P in place.

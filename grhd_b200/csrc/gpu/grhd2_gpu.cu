@@ -50,12 +50,13 @@ int vfail(std::string &err, int code, const char *fmt, va_list ap) {
 // kernel kinds of a step and their items-per-block
 enum Kind {
   K_RECON_X = 0, K_RIEMANN_X, K_RECON_Y, K_RIEMANN_Y, K_RECON_Z, K_RIEMANN_Z, K_CELL, K_FLUX_X, K_FLUX_Y, K_FLUX_Z,
-  K_STAGE, K_CELL_WIDE, NKIND
+  K_STAGE, K_CELL_WIDE, K_STAGE1D, NKIND
 };
 const int KIND_BS[NKIND] = {RECON_BS, RIEMANN_BS, RECON_BS, RIEMANN_BS, RECON_BS, RIEMANN_BS, CELL_BS,
-                            FUSED_FLUX_BS, FUSED_FLUX_BS, FUSED_FLUX_BS, STAGE_BLOCK, CELL_BS_WIDE};
+                            FUSED_FLUX_BS, FUSED_FLUX_BS, FUSED_FLUX_BS, STAGE_BLOCK, CELL_BS_WIDE,
+                            STAGE1D_BLOCK};
 const char *KIND_NAME[NKIND] = {"recon_x", "riemann_x", "recon_y", "riemann_y", "recon_z", "riemann_z",
-                                "cell_update", "flux_x", "flux_y", "flux_z", "stage", "cell_update"};
+                                "cell_update", "flux_x", "flux_y", "flux_z", "stage", "cell_update", "stage"};
 
 // ---- block tiles ------------------------------------------------------------------------
 unsigned ilog2(unsigned x) {
@@ -123,6 +124,7 @@ long long kind_items(const GridDev &G, int k) {
   // wide blocks keep the tile's 32 cells along i and take 8 along k
   if (k == K_CELL_WIDE) return G.nz > 1 ? tile_count(G.tiles[TILE_CELL], LB_CELL + 1, (unsigned)G.nz) * CELL_BS_WIDE : 0;
   if (k == K_STAGE) return stage_tiles(G) * STAGE_BLOCK;
+  if (k == K_STAGE1D) return stage_sd(G) == 0 ? (long long)((G.nx + STAGE1D_CELLS - 1) / STAGE1D_CELLS) * STAGE1D_BLOCK : 0;
   const int dir = k >= K_FLUX_X && k <= K_FLUX_Z ? k - K_FLUX_X + 1 : k / 2 + 1;
   if (!dir_active(G, dir)) return 0;
   unsigned nI, nJ, nK;
@@ -186,6 +188,7 @@ struct Group {
   int max_blocks_stage = 0;  // resident blocks of its persistent stage kernel (stage groups of 1D grids)
   int cell_dirs = 1;   // the most active directions of a member grid (cell kernel staging)
   bool cell_wide = false;  // FP64 cell update in 256-thread blocks
+  bool stage1d = false;  // the stage kernel's spread form (1D grids, small launches)
   bool stage = false;  // steps run the stage kernel (one launch per stage) instead of face and cell kernels
 };
 
@@ -386,6 +389,15 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
   return b->stage_request == GRHD2_STAGE_ON || grp.sd == 0;
 }
 
+// The stage kernel's spread form (stage1d.cuh) runs 1D groups while all their tiles together
+// are resident at once: 148 SMs x 2 blocks of 63 cells.  It shortens a tile's dependent chain
+// but keeps most of a block's threads idle in its last phases, so beyond one wave the 256-cell
+// tiles win.  Measured per step, graph replays, 256-cell tiles and spread form: tubes of 400
+// cells (WENO5 + HLLE, 7 tiles each) FP64 1 grid 81 and 55 us, 32 grids 86 and 62, 128 grids
+// 108 and 171; MP5 + HLLC 117 and 87, 125 and 94, 158 and 265; Michel 1024 (17 tiles) 70 and 43,
+// 8 grids 71 and 44, 32 grids 72 and 84; mixed tube 39 and 25, Michel 39 and 25.
+constexpr int STAGE1D_TILES_MAX = 148 * 2;
+
 // Whether a group's FP64 cell update runs in 256-thread blocks (cell.cuh): eight warps share
 // a table slice instead of four, which leaves L1 75 KB more and shared memory room to stage
 // up and u.  Measured on k tori of 400x1x200 (325 wide blocks each), us per stage, narrow and
@@ -519,6 +531,15 @@ int build_batch(grhd2_gpu_batch *b) {
       if (e != cudaSuccess) return bfail(b, GRHD2_ERR_CUDA, "persistent stage kernel occupancy: %s", cudaGetErrorString(e));
     }
   }
+  int tiles1d = 0;  // the groups of a step run side by side: their tiles share the GPU
+  for (const auto &grp : b->groups)
+    if (grp.stage && grp.sd == 0) tiles1d += grp.nb[K_STAGE1D];
+  for (auto &grp : b->groups) {
+    grp.stage1d = grp.stage && grp.sd == 0 && tiles1d <= STAGE1D_TILES_MAX;
+    if (!grp.stage1d) continue;
+    cudaError_t e = grp.mixed ? stage1d_setup<float, float>(grp.rec, grp.rs) : stage1d_setup<double, double>(grp.rec, grp.rs);
+    if (e != cudaSuccess) return bfail(b, GRHD2_ERR_CUDA, "1D stage kernel set-up: %s", cudaGetErrorString(e));
+  }
   BCUDA_TRY(b, cudaMallocAsync((void **)&b->d_bar, 4 * sizeof(unsigned), b->stream));
   BCUDA_TRY(b, cudaMemsetAsync(b->d_bar, 0, 4 * sizeof(unsigned), b->stream));
   // step mode
@@ -580,7 +601,11 @@ int enqueue_group_step(grhd2_gpu_batch *b, const Group &grp, cudaStream_t st) {
   if (grp.stage) {
     if (grp.nb[K_STAGE] <= 0) return 0;
     for (int mode = 1; mode <= 3; ++mode) {
-      if (grp.mixed)
+      if (grp.stage1d) {
+        const BlockMap *map = grp.d_map + grp.off[K_STAGE1D];
+        if (grp.mixed) launch_stage1d<float, float>(grp.rec, grp.rs, mode, b->d_grids, map, grp.nb[K_STAGE1D], st);
+        else launch_stage1d<double, double>(grp.rec, grp.rs, mode, b->d_grids, map, grp.nb[K_STAGE1D], st);
+      } else if (grp.mixed)
         launch_stage<float, float>(grp.sd, grp.rec, grp.rs, mode, b->d_grids, grp.d_map + grp.off[K_STAGE],
                                    grp.nb[K_STAGE], st);
       else

@@ -297,7 +297,14 @@ __device__ __forceinline__ void wavespeeds(const Phys &P, const R (&q)[NEQ], int
   wmin = rmin(rmin(rmin(R(0), e1), e2), e3);
 }
 
-// calc_hlle_fluxes, fluxes.f90:125-156
+// calc_hlle_fluxes, fluxes.f90:125-156; hlle_combine: one component from both sides
+template <class R>
+__device__ __forceinline__ R hlle_combine(R ap, R am, R fL, R fR, R uL, R uR) {
+  if (fabs(ap - am) < R(1.0e-14)) return R(0);
+  const R num = ap * fL - am * fR + ap * am * (uR - uL);
+  if (sizeof(R) == sizeof(float)) return num * (R(1) / (ap - am));  // as hlle: a reciprocal
+  return div_pos(num, ap - am);  // ap - am > 0 here (or NaN)
+}
 template <class R>
 __device__ __forceinline__ void hlle(const Phys &P, const R (&qL)[NEQ], const R (&qR)[NEQ], int dir,
                                      const FaceMetric<R> &m, R (&flux)[NEQ]) {

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "stage.cuh"
+#include "stage1d.cuh"
 #include "flux_launch.h"
 
 namespace grhd {
@@ -37,6 +38,34 @@ void launch_stage_sd(int rec, int rs, int mode, const GridDev *grids, const Bloc
   const void *fn = stage_kernel<SD, R, PT>(rec, rs);
   void *args[] = {(void *)&grids, (void *)&map, (void *)&mode};
   cudaLaunchKernel(fn, dim3((unsigned)nblocks), dim3(STAGE_BS), args, stage_smem_bytes<SD, R>(), s);
+}
+
+// the spread form for small launches of 1D grids (stage1d.cuh)
+static_assert(S1_BS == STAGE1D_BLOCK && S1_CELLS == STAGE1D_CELLS, "the host's tile geometry is the kernel's");
+template <int REC, class R, class PT>
+inline const void *stage1d_fn(int rs) {
+  return rs == RS_HLLC ? (const void *)k_stage1d<REC, RS_HLLC, R, PT> : (const void *)k_stage1d<REC, RS_HLLE, R, PT>;
+}
+template <class R, class PT>
+inline const void *stage1d_kernel(int rec, int rs) {
+  switch (rec) {
+    case REC_GODUNOV: return stage1d_fn<REC_GODUNOV, R, PT>(rs);
+    case REC_TVD: return stage1d_fn<REC_TVD, R, PT>(rs);
+    case REC_WENO3: return stage1d_fn<REC_WENO3, R, PT>(rs);
+    case REC_MP5: return stage1d_fn<REC_MP5, R, PT>(rs);
+    default: return stage1d_fn<REC_WENO5, R, PT>(rs);
+  }
+}
+template <class R, class PT>
+cudaError_t stage1d_setup(int rec, int rs) {
+  return cudaFuncSetAttribute(stage1d_kernel<R, PT>(rec, rs), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)S1Layout<R>::total);
+}
+template <class R, class PT>
+void launch_stage1d(int rec, int rs, int mode, const GridDev *grids, const BlockMap *map, int nblocks, cudaStream_t s) {
+  if (nblocks <= 0) return;
+  void *args[] = {(void *)&grids, (void *)&map, (void *)&mode};
+  cudaLaunchKernel(stage1d_kernel<R, PT>(rec, rs), dim3((unsigned)nblocks), dim3(S1_BS), args, S1Layout<R>::total, s);
 }
 
 }  // namespace grhd
