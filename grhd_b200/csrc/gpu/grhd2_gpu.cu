@@ -349,9 +349,24 @@ TuneKey tune_key(const Group &grp, const std::vector<GridDev> &hg, int dir) {
   return TuneKey{grp.mixed ? 1 : 0, grp.rec, grp.rs, hg[grp.members[0]].phys.sensor, dir, cls};
 }
 
-// default without tuning: the split kernels (recon at high occupancy, lean Riemann)
-constexpr int DEFAULT_VARIANT = GRHD2_FLUX_SPLIT;
-constexpr long long SPLIT_VAR_BELOW_FACES = 4LL * 148 * 4 * RECON_BS;  // four waves of per-face blocks
+// Default without tuning, by what wins for a launch's precision, Riemann solver and faces in a
+// direction.  Measured per step on batches of 1 to 32 tori 400x1x200 (80k faces each), 3D
+// tori of 48x24x24 to 256x128x128 and x-z grids of 256x128, us for split, split per variable
+// and fused:
+//   mixed: fused throughout (70 against 77-83 at 33k faces; tori 106 against 118-124 at 80k,
+//     1512 against 1910 at 2.6M; 3D torus MP5 + HLLC 3536 against 4267)
+//   FP64 HLLE: fused from 80k faces (167 against 189 and 181; 3006 against 3251 and 3614 at
+//     2.6M), split per variable at 33k (117 against 142 and 130) and 28k (186, 220, 190), whose
+//     one thread per face would leave SMs idle
+//   FP64 HLLC, whose fused form spills: split from 160k faces (356 against 397 and 364; 3D
+//     torus 8183 against 11315 and 9772), at 80k level (241, 237, 244), split per variable below
+//     (288, 253, 252 at 28k)
+constexpr long long FUSED_FROM_FACES = 60000, SPLIT_FROM_FACES = 120000;
+int default_variant(bool mixed, int rs, long long faces) {
+  if (mixed) return GRHD2_FLUX_FUSED;
+  if (rs == RS_HLLE) return faces >= FUSED_FROM_FACES ? GRHD2_FLUX_FUSED : GRHD2_FLUX_SPLIT_VAR;
+  return faces >= SPLIT_FROM_FACES ? GRHD2_FLUX_SPLIT : GRHD2_FLUX_SPLIT_VAR;
+}
 // Automatic step mode: the graph of stage kernels.  Measured on one B200 with 1024-cell 1D
 // grids, a graph replay takes 83-88 us per step and the persistent kernel 127-135 us: a
 // small grid is bound by the dependent arithmetic chain of one item per thread, not by
@@ -361,11 +376,9 @@ constexpr long long SPLIT_VAR_BELOW_FACES = 4LL * 148 * 4 * RECON_BS;  // four w
 FluxChoice choose_flux(const grhd2_gpu_batch *b, int gi, const Group &grp, const std::vector<GridDev> &hg, int dir) {
   auto f = b->forced.find({gi, dir});
   if (f != b->forced.end()) return f->second;
-  // untuned: one thread per (face, variable) for launches that one thread per face would
-  // leave short of the resident threads of the GPU
   long long faces = 0;
   for (int g : grp.members) faces += face_count(hg[g], dir);
-  FluxChoice c{faces < SPLIT_VAR_BELOW_FACES ? GRHD2_FLUX_SPLIT_VAR : DEFAULT_VARIANT, DEFAULT_TX};
+  FluxChoice c{default_variant(grp.mixed, grp.rs, faces), DEFAULT_TX};
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune.find(tune_key(grp, hg, dir));
@@ -2051,7 +2064,7 @@ int grhd2_gpu_batch_autotune(grhd2_gpu_batch *b, int reps, int *variants, int *t
     for (int d = 1; d <= 3 && !rc; ++d) {
       if (b->groups[gi].nb[K_FLUX_X + d - 1] <= 0) continue;
       float best = 0.0f;
-      FluxChoice best_c{DEFAULT_VARIANT, DEFAULT_TX};
+      FluxChoice best_c{GRHD2_FLUX_SPLIT, DEFAULT_TX};
       bool first = true;
       for (int v : {GRHD2_FLUX_SPLIT, GRHD2_FLUX_SPLIT_VAR, GRHD2_FLUX_FUSED}) {
         for (unsigned tx : {32u, 64u, 128u}) {
