@@ -409,6 +409,9 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
 // cells (WENO5 + HLLE, 7 tiles each) FP64 1 grid 81 and 55 us, 32 grids 86 and 62, 128 grids
 // 108 and 171; MP5 + HLLC 117 and 87, 125 and 94, 158 and 265; Michel 1024 (17 tiles) 70 and 43,
 // 8 grids 71 and 44, 32 grids 72 and 84; mixed tube 39 and 25, Michel 39 and 25.
+// Mixed HLLC groups keep the 256-cell tiles: in the spread form the compiler contracts other
+// multiply-add pairs of the FP32 HLLC, and its results would differ from the other kernels' by
+// 1e-7 on a tube (FP32 HLLE and the reconstructions are the same to the bit).
 constexpr int STAGE1D_TILES_MAX = 148 * 2;
 
 // Whether a group's FP64 cell update runs in 256-thread blocks (cell.cuh): eight warps share
@@ -548,7 +551,7 @@ int build_batch(grhd2_gpu_batch *b) {
   for (const auto &grp : b->groups)
     if (grp.stage && grp.sd == 0) tiles1d += grp.nb[K_STAGE1D];
   for (auto &grp : b->groups) {
-    grp.stage1d = grp.stage && grp.sd == 0 && tiles1d <= STAGE1D_TILES_MAX;
+    grp.stage1d = grp.stage && grp.sd == 0 && tiles1d <= STAGE1D_TILES_MAX && !(grp.mixed && grp.rs == RS_HLLC);
     if (!grp.stage1d) continue;
     cudaError_t e = grp.mixed ? stage1d_setup<float, float>(grp.rec, grp.rs) : stage1d_setup<double, double>(grp.rec, grp.rs);
     if (e != cudaSuccess) return bfail(b, GRHD2_ERR_CUDA, "1D stage kernel set-up: %s", cudaGetErrorString(e));

@@ -242,9 +242,10 @@ __device__ __forceinline__ void lower(const FaceMetric<R> &m, const R (&v)[3], R
   }
 }
 
-// calc_fluxes (F) and prim_to_cons_face (U) together: they share v_sq, h, W, v_cov
+// calc_fluxes (F) and prim_to_cons_face (U) together: they share v_sq, h, W, v_cov.  Without
+// the closing factor sqrt(gamma) of every component:
 template <class R>
-__device__ __forceinline__ void flux_and_cons(const Phys &P, const R (&q)[NEQ], int dir,
+__device__ __forceinline__ void flux_and_cons_bare(const Phys &P, const R (&q)[NEQ], int dir,
                                               const FaceMetric<R> &m, R (&f)[NEQ], R (&u)[NEQ]) {
   R v[3] = {q[EQ_VX], q[EQ_VY], q[EQ_VZ]}, vc[3];
   const R vsq = cap_velocity(m, v, R(P.v_max));
@@ -264,6 +265,11 @@ __device__ __forceinline__ void flux_and_cons(const Phys &P, const R (&q)[NEQ], 
   u[EQ_VX] = rhW2 * vc[0];
   u[EQ_VY] = rhW2 * vc[1];
   u[EQ_VZ] = rhW2 * vc[2];
+}
+template <class R>
+__device__ __forceinline__ void flux_and_cons(const Phys &P, const R (&q)[NEQ], int dir,
+                                              const FaceMetric<R> &m, R (&f)[NEQ], R (&u)[NEQ]) {
+  flux_and_cons_bare(P, q, dir, m, f, u);
 #pragma unroll
   for (int n = 0; n < NEQ; ++n) { f[n] = f[n] * m.sqg; u[n] = u[n] * m.sqg; }
 }

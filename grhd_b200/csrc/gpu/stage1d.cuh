@@ -11,14 +11,16 @@
 // memory:
 //   0  the grid's descriptor in one coalesced read; then, all in flight at once (cp.async),
 //      the primitives with their halo, the face table, up, u and con2prim's metric fields
-//   1  (face, variable, side): one interface state (reconstruct_1d_core)
+//   1  (face, variable): both interface states (reconstruct_1d_core)
 //   2  (face, side): physical flux, conserved state and wave speeds (HLLE), or one thread
 //      per face (HLLC); meanwhile the warps without a face evaluate the metric sources
 //   3  (face, variable): the HLLE combination
 //   4  (cell, variable): flux divergence, RK combination
 //   5  cell: con2prim
 // The expressions and their order are those of the other kernels, so FP64 results are the
-// same to the bit.  Measured: at STAGE1D_TILES_MAX in grhd2_gpu.cu.
+// same to the bit; in the mixed policy both states of a face are one thread's work, and the
+// HLLE sides stay without their sqrt(gamma) until they meet, so that the compiler contracts
+// the same multiply-add pairs as in the stage kernel (bit-identical with HLLE).  Measured: at STAGE1D_TILES_MAX in grhd2_gpu.cu.
 #pragma once
 
 #include "stage.cuh"
@@ -26,7 +28,7 @@
 namespace grhd {
 
 constexpr int S1_FACES = 64, S1_CELLS = S1_FACES - 1;  // whole warps of faces
-constexpr int S1_BS = 320;                             // two rounds of (face, variable, side)
+constexpr int S1_BS = 320;                             // one thread per (face, variable)
 constexpr int S1_BOX = S1_CELLS + 2 * STAGE_H;
 constexpr int S1_META = 13;  // con2prim's metric: gamma_ij, gamma^ij, sqrt(gamma)
 constexpr int S1_SIDE_WARPS = 2 * S1_FACES / 32;
@@ -51,23 +53,6 @@ struct S1Layout {
   static constexpr size_t flux = fu + stage_align(sizeof(R) * 2 * 12 * S1_FACES);
   static constexpr size_t total = flux + stage_align(sizeof(R) * NEQ * S1_FACES);
 };
-
-// one interface state from the window w[m * 1] (m = 0..5, cells face-2 .. face+3): side 0 the
-// left state, side 1 the right one (the mirrored window); recon_one's expressions
-template <int REC, class R>
-__device__ __forceinline__ R recon_side(int br, int lim, const R *w, int side) {
-  auto o = [&](int m) { return w[side ? 5 - m : m]; };
-  const R c = o(2);
-  if (br == BR_GODUNOV) return c;
-  if (REC == REC_TVD || (REC != REC_GODUNOV && br == BR_TVD_MC)) {
-    const R s1 = side ? w[2] : w[1], s2 = side ? w[3] : w[2], s3 = side ? w[4] : w[3];
-    const R h = R(0.5) * tvd_slope(s2 - s1, s3 - s2, REC == REC_TVD ? lim : LIM_MC);
-    return side ? c - h : c + h;
-  }
-  if (REC != REC_GODUNOV && br == BR_WENO3) return weno3(o(1), c, o(3));
-  if (REC == REC_MP5) return mp5(o(0), o(1), c, o(3), o(4));
-  return weno5(o(0), o(1), c, o(3), o(4));
-}
 
 // a table in shared memory as load_face_metric / load_face_frame read one (face f of n)
 template <class R>
@@ -194,29 +179,34 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
 
   // ---- 1. interface states ---------------------------------------------------------------------
   unsigned clamps = 0;
-#pragma unroll 1
-  for (int it = t; it < 2 * NEQ * S1_FACES; it += S1_BS) {
-    const int k = it / S1_FACES, f = it - k * S1_FACES;  // k: variable of the left, then of the right state
-    const int side = k >= NEQ, v = side ? k - NEQ : k, face = i0 - 1 + f;
-    if (f >= nf) continue;
-    int br = BR_GODUNOV;
-    if (REC != REC_GODUNOV) {
-      R rho[5], pr[5];
-      const bool sensor = P.sensor != 0;
+  {
+    const int v = t / S1_FACES, f = t - v * S1_FACES, face = i0 - 1 + f;
+    if (f < nf) {
+      int br = BR_GODUNOV;
+      if (REC != REC_GODUNOV) {
+        R rho[5], pr[5];
+        const bool sensor = P.sensor != 0;
 #pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        rho[m] = sensor ? s_p[EQ_DE * S1_BOX + f + m] : R(0);
-        pr[m] = sensor ? s_p[EQ_PR * S1_BOX + f + m] : R(0);
+        for (int m = 0; m < 5; ++m) {
+          rho[m] = sensor ? s_p[EQ_DE * S1_BOX + f + m] : R(0);
+          pr[m] = sensor ? s_p[EQ_PR * S1_BOX + f + m] : R(0);
+        }
+        br = branch_of<REC>(P, rho, pr, face, nx, 1);
       }
-      br = branch_of<REC>(P, rho, pr, face, nx, 1);
+      R s6[6], l, r;
+#pragma unroll
+      for (int m = 0; m < 6; ++m) s6[m] = (m >= lo && m <= hi) ? s_p[v * S1_BOX + f + m] : R(0);
+      recon_one<REC>(br, P.lim, s6, l, r);
+      if (v == EQ_DE || v == EQ_PR) {  // reconstruction.f90:647-655
+        const R fl = v == EQ_DE ? R(P.rho_floor) : R(P.p_floor);
+        if (f < S1_CELLS || face == nx)  // the tile that holds the upper cell counts
+          clamps = (unsigned)!(l >= fl) + (unsigned)!(r >= fl);
+        l = rmax(l, fl);
+        r = rmax(r, fl);
+      }
+      s_q[v * S1_FACES + f] = l;
+      s_q[(NEQ + v) * S1_FACES + f] = r;
     }
-    R r = recon_side<REC>(br, P.lim, s_p + v * S1_BOX + f, side);
-    if (v == EQ_DE || v == EQ_PR) {  // reconstruction.f90:647-655
-      const R fl = v == EQ_DE ? R(P.rho_floor) : R(P.p_floor);
-      if (f < S1_CELLS || face == nx) clamps += (unsigned)!(r >= fl);  // the tile that holds the upper cell counts
-      r = rmax(r, fl);
-    }
-    s_q[k * S1_FACES + f] = r;
   }
   count_add(G.cnt, CNT_RECON_CLAMP, clamps);
   __syncthreads();
@@ -245,7 +235,7 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
         R q[NEQ], ff[NEQ], uu[NEQ], wmin, wmax;
 #pragma unroll
         for (int v = 0; v < NEQ; ++v) q[v] = s_q[(side * NEQ + v) * S1_FACES + f];
-        flux_and_cons(P, q, 1, m, ff, uu);
+        flux_and_cons_bare(P, q, 1, m, ff, uu);
         wavespeeds(P, q, 1, m, wmin, wmax);
         R *o = s_fu + side * 12 * S1_FACES + f;
 #pragma unroll
@@ -286,7 +276,8 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
         const R ap = rmax(rmax(R(0), l[11 * S1_FACES]), r[11 * S1_FACES]);
         const R am = rmin(rmin(R(0), l[10 * S1_FACES]), r[10 * S1_FACES]);
         const R fL = l[v * S1_FACES], fR = r[v * S1_FACES], uL = l[(NEQ + v) * S1_FACES], uR = r[(NEQ + v) * S1_FACES];
-        flux = hlle_combine(ap, am, fL, fR, uL, uR);
+        const R sqg = s_t[FF_SQG * S1_FACES + f];
+        flux = hlle_combine(ap, am, fL * sqg, fR * sqg, uL * sqg, uR * sqg);
       }
       s_f[v * S1_FACES + f] = flux;
     }
