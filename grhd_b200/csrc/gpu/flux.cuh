@@ -162,6 +162,46 @@ __device__ __forceinline__ void recon_one(int br, int lim, const R (&s)[6], R &q
   if (REC == REC_WENO5) { qL = weno5(s[0], s[1], s[2], s[3], s[4]); qR = weno5(s[5], s[4], s[3], s[2], s[1]); return; }
 }
 
+// The Riemann flux of one face (resolve_riemann_problem) from its interface states, variable v
+// of side s at Q[(5 s + v) nq + fq], into F[v nf + f]; returns whether HLLC fell back to HLLE.
+template <int DIR, int RS, class R>
+__device__ __forceinline__ bool riemann_face(const GridDev &G, const Phys &P, const R *__restrict__ Q, long long nq,
+                                             long long fq, long long ft, R *__restrict__ F, long long nf, long long f) {
+  R qL[NEQ], qR[NEQ], flux[NEQ];
+#pragma unroll
+  for (int v = 0; v < NEQ; ++v) { qL[v] = Q[(long long)v * nq + fq]; qR[v] = Q[(long long)(5 + v) * nq + fq]; }
+  const R *T = face_table<R>(G, DIR - 1);
+  const long long ntab = G.nface[DIR - 1];
+  bool fb = false;
+  if (__ldg(&T[FF_ZERO * ntab + ft]) != R(0)) {
+#pragma unroll
+    for (int v = 0; v < NEQ; ++v) flux[v] = R(0);
+  } else {
+    const FaceMetric<R> m = load_face_metric<R>(T, ntab, ft);
+    if (RS == RS_HLLC) {
+      const FaceFrame<R> fr = load_face_frame<R>(T, ntab, ft);
+      fb = hllc_try(P, qL, qR, DIR, m, fr, flux);
+    } else {
+      fb = true;
+    }
+    if (fb) hlle(P, qL, qR, DIR, m, flux);  // the single HLLE call site
+  }
+#pragma unroll
+  for (int v = 0; v < NEQ; ++v) F[(long long)v * nf + f] = flux[v];
+  return fb;
+}
+// The same out of line.  The fused kernel takes its FP32 HLLC through this call: inlined behind
+// the reconstruction, the compiler contracts other multiply-add pairs of HLLC than in
+// k_riemann, and the mixed policy's results then depend on the kernel variant (5.6e-8 of the
+// state on a Kelvin-Helmholtz layer after 8 steps); called, both forms round alike, bit for
+// bit on 16 configurations, at the same speed (3D torus 3.52 ms a step against 3.54).
+template <int DIR, int RS, class R>
+__device__ __noinline__ bool riemann_face_call(const GridDev &G, const R *__restrict__ Q, long long nq, long long fq,
+                                               long long ft, R *__restrict__ F, long long nf, long long f) {
+  const Phys P = G.phys;
+  return riemann_face<DIR, RS, R>(G, P, Q, nq, fq, ft, F, nf, f);
+}
+
 // Batched launches: block b works on grid map[b].grid, tile map[b].first / blockDim.x.
 // Q layout per grid: Q[(side*5 + v) * nfaces + f], side 0 = q_L, 1 = q_R
 // Resident blocks per SM the register allocation must allow (256-thread recon blocks,
@@ -400,31 +440,14 @@ __device__ __forceinline__ void flux_item(const GridDev &G, unsigned a, unsigned
     sq[NEQ + v][threadIdx.x] = qR;
   }
   count_add(G.cnt, CNT_RECON_CLAMP, clamps);
-  R qL[NEQ], qR[NEQ], flux[NEQ];
-#pragma unroll
-  for (int v = 0; v < NEQ; ++v) { qL[v] = sq[v][threadIdx.x]; qR[v] = sq[NEQ + v][threadIdx.x]; }
   R *__restrict__ F = (R *)G.F[DIR - 1];
-  const R *T = face_table<R>(G, DIR - 1);
-  const long long ntab = G.nface[DIR - 1];
-  bool fb = false;
-  if (__ldg(&T[FF_ZERO * ntab + x.ft]) != R(0)) {
-#pragma unroll
-    for (int v = 0; v < NEQ; ++v) flux[v] = R(0);
-  } else {
-    const FaceMetric<R> m = load_face_metric<R>(T, ntab, x.ft);
-    if (RS == RS_HLLC) {
-      const FaceFrame<R> fr = load_face_frame<R>(T, ntab, x.ft);
-      fb = hllc_try(P, qL, qR, DIR, m, fr, flux);
-    } else {
-      fb = true;
-    }
-    if (fb) hlle(P, qL, qR, DIR, m, flux);
-  }
-#pragma unroll
-  for (int v = 0; v < NEQ; ++v) F[(long long)v * nf + f] = flux[v];
+  bool fb;
+  if constexpr (RS == RS_HLLC && sizeof(R) == sizeof(float))
+    fb = riemann_face_call<DIR, RS, R>(G, &sq[0][0], FLUX_BS, threadIdx.x, x.ft, F, nf, f);
+  else
+    fb = riemann_face<DIR, RS, R>(G, P, &sq[0][0], FLUX_BS, threadIdx.x, x.ft, F, nf, f);
   if (RS == RS_HLLC) count_add(G.cnt, CNT_HLLC_FALLBACK, fb ? 1u : 0u);
 }
-
 
 // Resident 128-thread blocks per SM for the fused kernel.  FP32 (mixed policy): 10 with
 // HLLE (48 registers; 8 and 12 measured 2.5 % and 0-1 % slower on the batched 2.5D torus),
@@ -466,27 +489,7 @@ __global__ void __launch_bounds__(128, riemann_min_blocks<RS, R>()) k_riemann(co
   R *__restrict__ F = (R *)G.F[DIR - 1];
   unsigned long long *cnt = G.cnt;
   const FaceIndex x = face_at<DIR>(G, a, b, c);
-  R qL[NEQ], qR[NEQ], flux[NEQ];
-#pragma unroll
-  for (int v = 0; v < NEQ; ++v) { qL[v] = Q[(long long)v * nf + f]; qR[v] = Q[(long long)(5 + v) * nf + f]; }
-  const R *T = face_table<R>(G, DIR - 1);
-  const long long ntab = G.nface[DIR - 1];
-  bool fb = false;
-  if (__ldg(&T[FF_ZERO * ntab + x.ft]) != R(0)) {
-#pragma unroll
-    for (int v = 0; v < NEQ; ++v) flux[v] = R(0);
-  } else {
-    const FaceMetric<R> m = load_face_metric<R>(T, ntab, x.ft);
-    if (RS == RS_HLLC) {
-      const FaceFrame<R> fr = load_face_frame<R>(T, ntab, x.ft);
-      fb = hllc_try(P, qL, qR, DIR, m, fr, flux);
-    } else {
-      fb = true;
-    }
-    if (fb) hlle(P, qL, qR, DIR, m, flux);  // the single HLLE call site
-  }
-#pragma unroll
-  for (int v = 0; v < NEQ; ++v) F[(long long)v * nf + f] = flux[v];
+  const bool fb = riemann_face<DIR, RS, R>(G, P, Q, nf, f, x.ft, F, nf, f);
   if (RS == RS_HLLC) count_add(cnt, CNT_HLLC_FALLBACK, fb ? 1u : 0u);
 }
 
