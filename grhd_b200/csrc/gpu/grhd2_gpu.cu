@@ -421,10 +421,13 @@ constexpr int STAGE1D_TILES_MAX = 148 * 2;
 // wide: k = 1 25.2 and 27.4, k = 2 38.0 and 36.2, k = 4 62.8 and 59.1, k = 12 157 and 146,
 // k = 32 405 and 376; 3D torus 256x128x128 635 and 568.  So wide blocks pay once they fill the
 // GPU (148 SMs x 4 resident blocks) more than once; below that the coarser blocks leave SMs
-// idle.  Every grid needs a k extent (other tiles share no slice).
+// idle.  Every grid needs a k extent (other tiles share no slice), and rounding the extents up
+// to 8 rows must not add more than 5 % threads over 4 rows (127x53x18: 24 rows against 20, 143 us
+// against 121).
 constexpr int WIDE_CELLS_FROM_BLOCKS = 148 * 4;
 bool use_wide_cells(const Group &grp, const std::vector<GridDev> &hg) {
   if (grp.mixed || grp.nb[K_CELL_WIDE] < WIDE_CELLS_FROM_BLOCKS) return false;
+  if (20LL * CELL_BS_WIDE * grp.nb[K_CELL_WIDE] > 21LL * CELL_BS * grp.nb[K_CELL]) return false;
   for (int g : grp.members)
     if (hg[g].nz == 1) return false;
   return true;
