@@ -686,8 +686,9 @@ __device__ inline double root_brent(double g1, double rho_floor, double D, doubl
   return -1.0;
 }
 // FP32 estimate of the residual and its derivative for E = tau + D scaled out:
-// f / E^2 and f' / E^2 at W, d = D / E, q = Q2 / E^2.  For g1 >= 1.9 and d <= 1.25 the factor V
-// is at most 2.1, so the error of f is below 1e-5 and that of f' below 1e-5 (1 + d W) / W^3.
+// f / E^2 and f' / E^2 at W, d = D / E, q = Q2 / E^2.  For g1 >= 1.9 and |d| <= 1.25 the term
+// V^2 (1 - 1/W^2) is at most 2 and V^2 at most 12, so the error of f is below 1.1e-5 (about 90
+// roundings of terms of order one) and that of f' below 1e-5 (1 + |d| W) / W^3.
 struct RootScreen {
   float g1, d, q;
   __device__ __forceinline__ void eval(float W, float &f, float &df) const {
@@ -740,43 +741,56 @@ __device__ inline double root_reference(double g1, double rho_floor, double D, d
 // The FP64 path's rare branches out of line: its kernels carry one copy beside the common
 // path.  (The mixed root finder inlines root_reference: a call there costs its stage kernel
 // 3 % on 1024-cell grids.)
-static __device__ __noinline__ double root_reference_call(double g1, double rho_floor, double D, double tau, double Q2,
-                                                          unsigned &flags) {
-  return root_reference(g1, rho_floor, D, tau, Q2, flags);
-}
 static __device__ __noinline__ double root_brent_call(double g1, double rho_floor, double D, double tau, double Q2) {
   return root_brent(g1, rho_floor, D, tau, Q2);
+}
+static __device__ __noinline__ double residual_call(double g1, double W, double D, double tau, double Q2) {
+  double f, df;
+  residual(g1, W, D, tau, Q2, f, df);
+  return f;
 }
 // The same root from fewer FP64 residuals.  The reference starts at the middle of
 // [1, max(1e3, 2 W_guess)] and bisects about ten times before Newton's step is accepted (12.4
 // residuals per torus cell, each four FP64 quotients).  A bisection's next iterate depends
 // on the residual only through two decisions -- bisect or Newton, and the sign of f -- so
-// while the FP32 estimate settles both with a margin (1e-4 E^2 against its error of 1e-5 E^2,
-// and an FP64 round-off of 1e-15 E^2), the bracket is halved in FP64 without evaluating the
-// residual in FP64.  From the first decision the estimate cannot settle on, the reference's
-// iteration continues unchanged: the iterates, and the root, are the same to the bit
-// (tests/test_gpu_root.py).  Measured with ncu on 8 tori 400x1x200, stage 1: FP64
-// instructions of the cell update 29.2e6 -> 17.9e6, 122 -> 111 us.
+// while the FP32 estimate settles both with a margin (2e-5 E^2 against its error below
+// 1.1e-5 E^2, and an FP64 round-off of 1e-15 E^2), the bracket is halved in FP64 without
+// evaluating the residual in FP64.  From the first decision the estimate cannot settle on,
+// the reference's iteration continues unchanged: the iterates, and the root, are the same to
+// the bit (tests/test_gpu_root.py).  Operands the estimate does not cover join that
+// iteration at its start: the lanes of a warp share one loop, so a few such cells in a
+// floored region do not add a second pass to it (with a separate loop for them, 3D tori of
+// 48 rows stepped slower than without the estimate).  Measured with ncu on 8 tori 400x1x200,
+// stage 1: FP64 instructions of the cell update 29.2e6 -> 17.9e6, 122 -> 111 us.
 __device__ inline double root_safe_newton(double g1, double rho_floor, double D, double tau, double Q2, unsigned &flags) {
   const float Ef = (float)(tau + D), Df = (float)D, Qf = (float)Q2;
-  // V is finite at W = 1 for these operands, so f(1) = V^2 (1 - 1/1) - Q2 = -Q2
-  if (!(Ef > 1.0e-12f && Ef < 1.0e12f && Df > 0.0f && Df <= 1.25f * Ef && Qf < 1.0e24f && Q2 >= 0.0 && g1 >= 1.9))
-    return root_reference_call(g1, rho_floor, D, tau, Q2, flags);
-  if (Q2 < 1.0e-14) return 1.0;
+  const float aE = fabsf(Ef);  // E < 0 (a state gone bad) too: f depends on E^2 and D / E
+  const bool sane = aE > 1.0e-12f && aE < 1.0e12f && fabsf(Df) <= 1.25f * aE && Qf < 1.0e24f && Q2 >= 0.0 && g1 >= 1.9;
+  // NaN operands (a cell that went bad in this stage): both ends of the bracket are NaN and
+  // alike in sign, which the reference takes for "no sign change"
+  if (!sane && (Q2 != Q2 || tau + D != tau + D)) return -1.0;
+  // V is finite at W = 1 for sane operands, so f(1) = V^2 (1 - 1/1) - Q2 = -Q2
+  const double f_low = sane ? -Q2 : residual_call(g1, 1.0, D, tau, Q2);
+  if (fabs(f_low) < 1.0e-14) return 1.0;
   const double x2 = rmax(1.0e3, (sqrt(Q2) + D) / rmax(D, rho_floor) * 2.0);
-  const float iE = __fdividef(1.0f, Ef);
+  double x_low = 1.0, x_high = x2, root = 0.5 * (1.0 + x2), dx = fabs(x2 - 1.0), dx_old = dx;
+  const float iE = __fdividef(1.0f, Ef), x2f = (float)x2;
   const RootScreen scr{(float)g1, Df * iE, Qf * iE * iE};
-  float fs, dfs;
-  scr.eval((float)x2, fs, dfs);  // f(x2) certainly positive and not "zero": the bracket is [1, x2]
-  if (!((float)x2 < 1.0e5f && fs > 1.0e-4f && fs * Ef * Ef > 2.0e-14f))
-    return root_reference_call(g1, rho_floor, D, tau, Q2, flags);
-  double x_low = 1.0, x_high = x2, root = 0.5 * (1.0 + x2), dx = x2 - 1.0, dx_old = dx, f, df;
+  const bool screened = sane && x2f < 1.0e5f;
+  float fs = 0.0f, dfs = 0.0f;
+  if (screened) scr.eval(x2f, fs, dfs);
+  if (!(fs > 2.0e-5f && fs * Ef * Ef > 2.0e-14f)) {  // else f(x2) is certainly positive and not "zero"
+    const double f_high = residual_call(g1, x2, D, tau, Q2);
+    if (fabs(f_high) < 1.0e-14) return x2;
+    if (sgn1(f_low) * sgn1(f_high) > 0.0) return -1.0;
+    if (!(f_low < 0.0)) { x_high = 1.0; x_low = x2; }
+  }
   bool sign_open = false;  // the sign of f at root is not in the bracket yet
   int it = 0;
-  {
+  if (screened) {
     float of = (float)dx_old, nf = of;  // dx_old, dx
     scr.eval((float)root, fs, dfs);
-    while (nf > 1.0e-2f && fabsf(2.0f * fs) > 1.01f * fabsf(of * dfs) + 2.0e-4f) {  // bisection for certain
+    while (nf > 1.0e-2f && fabsf(2.0f * fs) > 1.01f * fabsf(of * dfs) + 1.0e-4f) {  // bisection for certain
       dx_old = dx;
       dx = 0.5 * (x_high - x_low);
       root = x_low + dx;
@@ -784,11 +798,12 @@ __device__ inline double root_safe_newton(double g1, double rho_floor, double D,
       of = nf;
       nf = (float)dx;
       scr.eval((float)root, fs, dfs);
-      sign_open = !(fabsf(fs) > 1.0e-4f);
+      sign_open = !(fabsf(fs) > 2.0e-5f);
       if (sign_open) break;
       if (fs < 0.0f) x_low = root; else x_high = root;
     }
   }
+  double f, df;
   for (;; ++it) {
     residual(g1, root, D, tau, Q2, f, df);
     if (sign_open) { if (f < 0.0) x_low = root; else x_high = root; }

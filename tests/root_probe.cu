@@ -56,7 +56,7 @@ __device__ __forceinline__ unsigned long long mix(unsigned long long h) {
 
 // kind 0: states of rho, p, v (densities over 40 binades, v up to 1 - 1e-5); 1: the same with
 // every conserved value off by up to 3 (no physical state behind it); 2: near the tests'
-// edges (Q2 ~ 1e-14, E ~ 1e-12 and 1e12, D ~ 1.25 E); 3: zeros, negative and infinite values
+// edges (Q2 ~ 1e-14, E ~ 1e-12 and 1e12, D ~ 1.25 E); 3: zeros, negative and infinite values; 4: E < 0
 __global__ void check(long long n, unsigned long long seed, int kind) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -82,6 +82,10 @@ __global__ void check(long long n, unsigned long long seed, int kind) {
     if (u() < 0.5) tau = odd[(mix(h) >> 8) & 7];
     if (u() < 0.5) Q2 = odd[(mix(h) >> 16) & 7];
   }
+  if (kind == 4) {  // E = tau + D < 0
+    tau = -D * (1.0 + (u() < 0.5 ? 4.0 * u() : exp2(-20.0 * u())));
+    Q2 = fmax(0.0, (tau + D) * (tau + D) - (u() < 0.5 ? D * D : 0.0)) * u();
+  }
   unsigned fa = 0, fb = 0;
   int ne = 0;
   const double a = root_safe_newton(g1, 1.0e-10, D, tau, Q2, fa), b = plain(g1, 1.0e-10, D, tau, Q2, fb, ne);
@@ -93,7 +97,7 @@ __global__ void check(long long n, unsigned long long seed, int kind) {
 
 int main() {
   const long long n = 1LL << 23;
-  for (int kind = 0; kind < 4; ++kind) {
+  for (int kind = 0; kind < 5; ++kind) {
     unsigned long long c[3], z = 0;
     cudaMemcpyToSymbol(g_tests, &z, 8);
     cudaMemcpyToSymbol(g_bad, &z, 8);

@@ -2,9 +2,9 @@
 outcome an FP32 estimate settles; its iterates and root must stay those of the reference's
 iteration (equations.f90:249-340) to the bit.
 
-tests/root_probe.cu includes the shipped header and compares both on 3.4e7 seeded states:
+tests/root_probe.cu includes the shipped header and compares both on 4.2e7 seeded states:
 physical ones, ones with no physical state behind them, ones at the edges of the estimate's
-range, and zero, negative and infinite input.
+range, zero, negative and infinite input, and negative total energy.
 """
 import os
 import re
@@ -29,5 +29,5 @@ def test_screened_root_is_the_reference_root():
                         "-I", INC, "-o", exe, SRC], check=True, capture_output=True, text=True)
         out = subprocess.run([exe], check=True, capture_output=True, text=True, timeout=120).stdout
     rows = re.findall(r"kind (\d) samples (\d+) bad (\d+)", out)
-    assert len(rows) == 4, out
+    assert len(rows) == 5, out
     assert all(int(bad) == 0 for _, _, bad in rows), out
