@@ -59,17 +59,18 @@ GRHD_STAGE_EXTERN(0, float)
 GRHD_STAGE_EXTERN(2, float)
 GRHD_STAGE_EXTERN(3, float)
 #undef GRHD_STAGE_EXTERN
-// its spread form for small launches of 1D grids (stage1d.cuh): tiles of STAGE1D_CELLS cells
+// its spread form for small launches of 1D grids (stage1d.cuh): tiles of STAGE1D_CELLS cells;
+// advance: the launch also advances its grids' clocks (the last stage's)
 constexpr int STAGE1D_CELLS = 63;
 constexpr int STAGE1D_BLOCK = 320;
 template <class R, class PT>
 cudaError_t stage1d_setup(int rec, int rs);
 template <class R, class PT>
-void launch_stage1d(int rec, int rs, int mode, const GridDev *grids, const BlockMap *map, int nblocks, cudaStream_t s);
+void launch_stage1d(int rec, int rs, int mode, int advance, const GridDev *grids, const BlockMap *map, int nblocks, cudaStream_t s);
 extern template cudaError_t stage1d_setup<double, double>(int, int);
 extern template cudaError_t stage1d_setup<float, float>(int, int);
-extern template void launch_stage1d<double, double>(int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
-extern template void launch_stage1d<float, float>(int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
+extern template void launch_stage1d<double, double>(int, int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
+extern template void launch_stage1d<float, float>(int, int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
 // sets the kernel's dynamic shared-memory limit; call before the first launch (outside a
 // stream capture)
 template <class R, class PT>

@@ -409,7 +409,9 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
 // tiles win.  Measured per step, graph replays, 256-cell tiles and spread form: tubes of 400
 // cells (WENO5 + HLLE, 7 tiles each) FP64 1 grid 81 and 55 us, 32 grids 86 and 62, 128 grids
 // 108 and 171; MP5 + HLLC 117 and 87, 125 and 94, 158 and 265; Michel 1024 (17 tiles) 70 and 43,
-// 8 grids 71 and 44, 32 grids 72 and 84; mixed tube 39 and 25, Michel 39 and 25.
+// 8 grids 71 and 44, 32 grids 72 and 84; mixed tube 39 and 25, Michel 39 and 25.  With the
+// launches overlapped (programmatic serialisation) and the clocks advanced in the last stage
+// the spread form's figures are 51 (tube FP64), 83 (HLLC), 41 (Michel), 19 and 21 us (mixed).
 // Mixed HLLC groups keep the 256-cell tiles: in the spread form the compiler contracts other
 // multiply-add pairs of the FP32 HLLC, and its results would differ from the other kernels' by
 // 1e-7 on a tube (FP32 HLLE and the reconstructions are the same to the bit).
@@ -616,15 +618,16 @@ int enqueue_cells(grhd2_gpu_batch *b, const Group &grp, cudaStream_t st) {
 }
 
 // the three SSP-RK3 stages of one scheme group (its grids depend on no other group's)
-int enqueue_group_step(grhd2_gpu_batch *b, const Group &grp, cudaStream_t st) {
+int enqueue_group_step(grhd2_gpu_batch *b, const Group &grp, bool advance, cudaStream_t st) {
   int rc;
   if (grp.stage) {
     if (grp.nb[K_STAGE] <= 0) return 0;
     for (int mode = 1; mode <= 3; ++mode) {
+      const int adv = advance && mode == 3;
       if (grp.stage1d) {
         const BlockMap *map = grp.d_map + grp.off[K_STAGE1D];
-        if (grp.mixed) launch_stage1d<float, float>(grp.rec, grp.rs, mode, b->d_grids, map, grp.nb[K_STAGE1D], st);
-        else launch_stage1d<double, double>(grp.rec, grp.rs, mode, b->d_grids, map, grp.nb[K_STAGE1D], st);
+        if (grp.mixed) launch_stage1d<float, float>(grp.rec, grp.rs, mode, adv, b->d_grids, map, grp.nb[K_STAGE1D], st);
+        else launch_stage1d<double, double>(grp.rec, grp.rs, mode, adv, b->d_grids, map, grp.nb[K_STAGE1D], st);
       } else if (grp.mixed)
         launch_stage<float, float>(grp.sd, grp.rec, grp.rs, mode, b->d_grids, grp.d_map + grp.off[K_STAGE],
                                    grp.nb[K_STAGE], st);
@@ -683,13 +686,18 @@ int enqueue_step(grhd2_gpu_batch *b, bool branches = false) {
     BCUDA_TRY(b, cudaEventRecord(b->fork, b->stream));
     for (int g = 1; g < ng; ++g) BCUDA_TRY(b, cudaStreamWaitEvent(b->lanes[g - 1], b->fork, 0));
   }
+  // Where every group runs the spread stage kernel, its last stage advances the clocks: a
+  // launch less (the 256-cell tiles, whose launches are larger, lost 5 % by doing the same).
+  bool advance = true;
+  for (const auto &grp : b->groups) advance = advance && grp.stage1d;
   for (int g = 0; g < ng; ++g)
-    if (int rc = enqueue_group_step(b, b->groups[g], branches && g > 0 ? b->lanes[g - 1] : b->stream)) return rc;
+    if (int rc = enqueue_group_step(b, b->groups[g], advance, branches && g > 0 ? b->lanes[g - 1] : b->stream)) return rc;
   if (branches)
     for (int g = 1; g < ng; ++g) {
       BCUDA_TRY(b, cudaEventRecord(b->lane_done[g - 1], b->lanes[g - 1]));
       BCUDA_TRY(b, cudaStreamWaitEvent(b->stream, b->lane_done[g - 1], 0));
     }
+  if (advance) return 0;
   const int n = (int)b->m.size();
   k_advance_clocks<<<nblocks(n, 128), 128, 0, b->stream>>>(b->d_grids, n);
   return blaunch_check(b, "advance_clocks");

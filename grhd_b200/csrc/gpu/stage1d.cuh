@@ -106,8 +106,11 @@ struct S1Prims {
 
 template <int REC, int RS, class R, class PT>
 __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
-    k_stage1d(const GridDev *__restrict__ grids, const BlockMap *__restrict__ map, int mode) {
+    k_stage1d(const GridDev *__restrict__ grids, const BlockMap *__restrict__ map, int mode, int advance) {
   extern __shared__ __align__(16) unsigned char s1[];
+  // the next stage's blocks may take their places now: they read map and descriptor, which no
+  // kernel writes, and wait below for this launch to complete
+  asm volatile("griddepcontrol.launch_dependents;");
   using L = S1Layout<R>;
   double *s_up = (double *)(s1 + L::up), *s_u = (double *)(s1 + L::u), *s_meta = (double *)(s1 + L::meta);
   double *s_src = (double *)(s1 + L::src), *s_cs = (double *)(s1 + L::cs);
@@ -123,6 +126,7 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
     const unsigned *src = (const unsigned *)&grids[bm.grid];
     for (int w = t; w < words; w += S1_BS) ((unsigned *)(s1 + L::desc))[w] = __ldg(&src[w]);
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous launch is complete, its writes visible
   __syncthreads();
   const GridDev &G = *(const GridDev *)(s1 + L::desc);
   const GridClock ck = *G.clock;
@@ -309,6 +313,8 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
     }
   }
   __syncthreads();
+
+  if (advance && t == S1_BS - 1) advance_when_done(G.clock, (unsigned)((nx + S1_CELLS - 1) / S1_CELLS));
 
   // ---- 5. con2prim ---------------------------------------------------------------------------------
   if (t >= nc) return;

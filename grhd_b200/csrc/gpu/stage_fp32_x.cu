@@ -5,5 +5,5 @@ namespace grhd {
 template cudaError_t stage_setup_sd<0, float, float>(int, int);
 template void launch_stage_sd<0, float, float>(int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
 template cudaError_t stage1d_setup<float, float>(int, int);
-template void launch_stage1d<float, float>(int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
+template void launch_stage1d<float, float>(int, int, int, int, const GridDev *, const BlockMap *, int, cudaStream_t);
 }  // namespace grhd

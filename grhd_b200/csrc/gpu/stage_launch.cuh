@@ -61,11 +61,24 @@ cudaError_t stage1d_setup(int rec, int rs) {
   return cudaFuncSetAttribute(stage1d_kernel<R, PT>(rec, rs), cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)S1Layout<R>::total);
 }
+// Launched with programmatic stream serialisation: the next stage's launch and descriptor
+// reads overlap this stage (measured per step: see STAGE1D_TILES_MAX).
 template <class R, class PT>
-void launch_stage1d(int rec, int rs, int mode, const GridDev *grids, const BlockMap *map, int nblocks, cudaStream_t s) {
+void launch_stage1d(int rec, int rs, int mode, int advance, const GridDev *grids, const BlockMap *map, int nblocks,
+                    cudaStream_t s) {
   if (nblocks <= 0) return;
-  void *args[] = {(void *)&grids, (void *)&map, (void *)&mode};
-  cudaLaunchKernel(stage1d_kernel<R, PT>(rec, rs), dim3((unsigned)nblocks), dim3(S1_BS), args, S1Layout<R>::total, s);
+  void *args[] = {(void *)&grids, (void *)&map, (void *)&mode, (void *)&advance};
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)nblocks);
+  cfg.blockDim = dim3(S1_BS);
+  cfg.dynamicSmemBytes = S1Layout<R>::total;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelExC(&cfg, stage1d_kernel<R, PT>(rec, rs), args);
 }
 
 }  // namespace grhd

@@ -55,6 +55,7 @@ struct GridClock {
   double t, final_time, dt_cfl, dt_explicit;
   long long steps, max_steps;
   int mode, active;
+  unsigned done;  // blocks of the running last stage that have finished with the grid (advance_when_done)
 };
 __host__ __device__ __forceinline__ double clock_dt(const GridClock &c) {
   if (c.mode == 0) return c.dt_explicit;
@@ -72,6 +73,17 @@ __device__ __forceinline__ void advance_clock(GridClock *c) {
   } else {
     c->steps += 1;
   }
+}
+
+// The clock's advance inside the last stage's kernel: called by one thread of each of the
+// grid's nblk blocks, after a barrier that follows the block's reads of the clock.  The last
+// block to come advances it; the others have read it by then.
+__device__ __forceinline__ void advance_when_done(GridClock *c, unsigned nblk) {
+  __threadfence();
+  if (atomicAdd(&c->done, 1u) != nblk - 1u) return;
+  __threadfence();
+  c->done = 0u;
+  advance_clock(c);
 }
 
 // Loads of the primitives.  Within one stage kernel they are read-only (the non-coherent
