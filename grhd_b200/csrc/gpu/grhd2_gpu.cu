@@ -414,7 +414,7 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
 // the spread form's figures are 51 (tube FP64), 83 (HLLC), 41 (Michel), 19 and 21 us (mixed).
 // Mixed HLLC groups keep the 256-cell tiles: in the spread form the compiler contracts other
 // multiply-add pairs of the FP32 HLLC, and its results would differ from the other kernels' by
-// 1e-7 on a tube (FP32 HLLE and the reconstructions are the same to the bit).
+// 1e-7 on a tube (FP32 HLLE fluxes and reconstructions are the same to the bit).
 constexpr int STAGE1D_TILES_MAX = 148 * 2;
 
 // Whether a group's FP64 cell update runs in 256-thread blocks (cell.cuh): eight warps share
@@ -1337,10 +1337,10 @@ static int copy_prims_in(grhd2_gpu *h, const double *p) {
 // can address, and it is small: the layout kernel then reads or writes it itself, without a
 // copy beside it.  NULL for other memory and larger arrays.  Measured, copy and direct: per
 // grid and call (8 grids in a loop) 15 KB 9.0 and 6.3 us, 80 KB 10.8 and 6.3, 160 KB 12.2 and
-// 10.3, 781 KB 26 and 22; 16 grids pipelined on four streams 80 KB 307 and 247 us, 195 KB 341 and
-// 347, but 781 KB 617 and 864: a large array's PCIe time holds SMs that the other streams'
-// steps want, so those keep the copy engines.
-constexpr size_t DIRECT_COPY_BYTES = (size_t)1 << 18;
+// 10.3, 781 KB 26 and 22; 12 to 16 grids pipelined on four streams 80 KB 289 and 209 us, 121 KB
+// 238 and 221, but 252 KB 185 and 207, 781 KB 617 and 864: a larger array's PCIe time holds SMs
+// that the other streams' steps want, so those keep the copy engines.
+constexpr size_t DIRECT_COPY_BYTES = (size_t)1 << 17;
 static double *device_view(const grhd2_gpu *h, const double *host) {
   const size_t bytes = h->n_interior * sizeof(double);
   if (bytes > DIRECT_COPY_BYTES) return nullptr;

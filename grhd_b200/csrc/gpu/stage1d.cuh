@@ -20,7 +20,8 @@
 // The expressions and their order are those of the other kernels, so FP64 results are the
 // same to the bit; in the mixed policy both states of a face are one thread's work, and the
 // HLLE sides stay without their sqrt(gamma) until they meet, so that the compiler contracts
-// the same multiply-add pairs as in the stage kernel (bit-identical with HLLE).  Measured: at STAGE1D_TILES_MAX in grhd2_gpu.cu.
+// the same multiply-add pairs as in the stage kernel: the FP32 fluxes of HLLE are the same to
+// the bit, con2prim's FP64 may differ in its last bits.  Measured: at STAGE1D_TILES_MAX in grhd2_gpu.cu.
 #pragma once
 
 #include "stage.cuh"
@@ -304,7 +305,10 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
         G.U[k] = up;  // u = up (grhd2.f90:232)
         nv = up + rhs * dt;
       } else if (mode == 2) {
-        nv = 0.75 * s_u[v * S1_CELLS + a] + 0.25 * (up + rhs * dt);
+        const double u = s_u[v * S1_CELLS + a], x = up + rhs * dt;
+        // mixed: the multiply-add pair the compiler contracts in the other kernels, spelled out
+        if (sizeof(PT) == sizeof(float)) nv = fma(0.75, u, 0.25 * x);
+        else nv = 0.75 * u + 0.25 * x;
       } else {
         nv = (s_u[v * S1_CELLS + a] + 2.0 * (up + rhs * dt)) / 3.0;
       }

@@ -1,5 +1,5 @@
 """Copies of the state between host and device by every route: pageable memory, page-locked
-memory small enough for the layout kernels to address it themselves (256 KiB), and larger
+memory small enough for the layout kernels to address it themselves (128 KiB), and larger
 page-locked memory, with arrays that do and do not start on a 16-byte boundary.  All must
 move the same bytes.  The ghosted primitives'
 upload, which skips the ghost planes, is held to the oracle by test_gpu_cases.py (the schemes
@@ -22,7 +22,7 @@ def _ptr(t, offset):
     return C.cast(t.data_ptr() + 8 * offset, C.POINTER(C.c_double))
 
 
-@pytest.mark.parametrize("nx", [5, 256, 257, 6553, 6554, 40000])  # 6553 cells: the last below 256 KiB
+@pytest.mark.parametrize("nx", [5, 256, 257, 3276, 3277, 40000])  # 3276 cells: the last below 128 KiB
 @pytest.mark.parametrize("offset", [0, 1])
 def test_state_copies_agree(nx, offset):
     import torch
