@@ -146,11 +146,12 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
       const int v = pos / S1_BOX, i = i0 - STAGE_H + (pos - v * S1_BOX);
       if (i >= 1 && i <= nx && i >= ia && i <= ib) cp_async<sizeof(PT)>(&s_p[pos], &Pin[v * pl + (i - 1)]);
     }
-    if (t < 2 * STAGE_H) {  // boundary fill of the cells outside the domain
+    if (t < 2 * STAGE_H) {  // boundary fill of the cells outside the domain (coherent: Pin was written
+                            // while this block was resident)
       const int i = t < STAGE_H ? i0 - STAGE_H + t : i0 + nc + (t - STAGE_H);
       if ((i < 1 || i > nx) && i >= ia && i <= ib) {
         double b[NEQ];
-        load_cell<1>(Pin, G, i, 1, 1, b);
+        load_cell<1, true>(Pin, G, i, 1, 1, b);
 #pragma unroll
         for (int v = 0; v < NEQ; ++v) s_p[v * S1_BOX + (i - (i0 - STAGE_H))] = R(b[v]);
       }

@@ -86,14 +86,21 @@ __device__ __forceinline__ void advance_when_done(GridClock *c, unsigned nblk) {
   advance_clock(c);
 }
 
-// Loads of the primitives.  Within one stage kernel they are read-only (the non-coherent
-// read-only path is safe); the persistent step kernel writes them between its phases, so
-// its translation units read them through L2 (ld.global.cg), coherent across blocks.
+// Loads of the primitives.  The non-coherent read-only path (ld.global.nc) wants them unmodified
+// for a kernel's whole lifetime.  A stage kernel launched after its predecessor has ended gives
+// that; two kinds do not and read through L2 (ld.global.cg): the persistent step kernel, which
+// writes primitives between its phases (its translation units define GRHD_PERSISTENT_TU), and
+// kernels launched with early dependents (stage1d.cuh), whose blocks are resident while the
+// previous stage still writes what they will read (COHERENT below).
 #ifdef GRHD_PERSISTENT_TU
 #define GRHD_LDP(ptr) __ldcg(ptr)
 #else
 #define GRHD_LDP(ptr) __ldg(ptr)
 #endif
+template <bool COHERENT, class PT>
+__device__ __forceinline__ double ld_prim_at(const PT *ptr) {
+  return (double)(COHERENT ? __ldcg(ptr) : GRHD_LDP(ptr));
+}
 
 // Division by a grid extent with a multiply-high and a shift (Granlund and Montgomery,
 // "Division by invariant integers using multiplication", 1994): for d >= 1 with
@@ -201,11 +208,11 @@ __device__ __forceinline__ double ld_prim(const PT *__restrict__ P, const GridDe
   const unsigned c = cell_index(G, i, j, k);
   return (double)GRHD_LDP(&P[v * G.pplane + c]);
 }
-template <class PT>
+template <bool COHERENT = false, class PT>
 __device__ __forceinline__ void ld_cell(const PT *__restrict__ P, const GridDev &G, int i, int j, int k, double (&q)[NEQ]) {
   const unsigned c = cell_index(G, i, j, k);
 #pragma unroll
-  for (int v = 0; v < NEQ; ++v) q[v] = (double)GRHD_LDP(&P[v * G.pplane + c]);
+  for (int v = 0; v < NEQ; ++v) q[v] = ld_prim_at<COHERENT>(&P[v * G.pplane + c]);
 }
 __device__ __forceinline__ int wrap(int i, int n) {  // periodic (whole-array statements per g) == modular
   int r = (i - 1) % n;
@@ -216,12 +223,13 @@ __device__ __forceinline__ void jet_ambient(const GridDev &G, double (&q)[NEQ]) 
   q[EQ_DE] = G.jet[0]; q[EQ_PR] = G.jet[1]; q[EQ_VX] = 0.0; q[EQ_VY] = 0.0; q[EQ_VZ] = G.jet[2];
 }
 
-// Value of cell (i,j,k) where only the DIR index may lie outside [1, n_DIR].
-template <int DIR, class PT>
+// Value of cell (i,j,k) where only the DIR index may lie outside [1, n_DIR].  COHERENT: the
+// primitives may have been written while this kernel was already resident.
+template <int DIR, bool COHERENT = false, class PT>
 __device__ __forceinline__ void load_cell(const PT *__restrict__ P, const GridDev &G, int i, int j, int k, double (&q)[NEQ]) {
   const int n = DIR == 1 ? G.nx : (DIR == 2 ? G.ny : G.nz);
   const int idx = DIR == 1 ? i : (DIR == 2 ? j : k);
-  if (idx >= 1 && idx <= n) { ld_cell(P, G, i, j, k, q); return; }
+  if (idx >= 1 && idx <= n) { ld_cell<COHERENT>(P, G, i, j, k, q); return; }
   const int cs = G.case_id;
   if (idx == -G.ng) {  // never written by the boundary loops (see header)
     if (cs == 5) { jet_ambient(G, q); return; }
@@ -239,14 +247,14 @@ __device__ __forceinline__ void load_cell(const PT *__restrict__ P, const GridDe
   if (DIR == 1) {
     switch (cs) {
       case 1: case 2: case 3:  // zero-gradient outflow, conditions.f90:795-798
-        ld_cell(P, G, lo ? 1 : G.nx, j, k, q); return;
+        ld_cell<COHERENT>(P, G, lo ? 1 : G.nx, j, k, q); return;
       case 4: case 6:  // periodic, conditions.f90:809-811
-        ld_cell(P, G, wrap(i, G.nx), j, k, q); return;
+        ld_cell<COHERENT>(P, G, wrap(i, G.nx), j, k, q); return;
       case 5:  // reflecting axis / ambient, conditions.f90:838-848
-        if (lo) { ld_cell(P, G, g, j, k, q); q[EQ_VX] = -q[EQ_VX]; } else jet_ambient(G, q);
+        if (lo) { ld_cell<COHERENT>(P, G, g, j, k, q); q[EQ_VX] = -q[EQ_VX]; } else jet_ambient(G, q);
         return;
       case 7:  // copy inside, analytic injector outside, conditions.f90:872-883
-        if (lo) ld_cell(P, G, 1, j, k, q);
+        if (lo) ld_cell<COHERENT>(P, G, 1, j, k, q);
         else {
 #pragma unroll
           for (int v = 0; v < NEQ; ++v)
@@ -255,7 +263,7 @@ __device__ __forceinline__ void load_cell(const PT *__restrict__ P, const GridDe
         return;
       case 8:  // dust, conditions.f90:896-907
         if (lo) {
-          ld_cell(P, G, 1, j, k, q);
+          ld_cell<COHERENT>(P, G, 1, j, k, q);
           q[EQ_DE] = rmax(q[EQ_DE], G.rho_floor);
           q[EQ_PR] = rmax(q[EQ_PR], G.p_floor);
           q[EQ_VX] = rmin(0.0, q[EQ_VX]);
@@ -266,7 +274,7 @@ __device__ __forceinline__ void load_cell(const PT *__restrict__ P, const GridDe
         return;
       default: {  // 9-12: shift-aware radial outflow, conditions.f90:916-938, :951-973, :1007-1026
         const int src = lo ? 1 : G.nx;
-        ld_cell(P, G, src, j, k, q);
+        ld_cell<COHERENT>(P, G, src, j, k, q);
         const double d_in = q[EQ_DE];
         const double va = G.centre[(long long)CF_VA * G.nij + (src - 1) + (long long)G.nx * (j - 1)];
         q[EQ_DE] = rmax(q[EQ_DE], G.rho_floor);
@@ -279,18 +287,18 @@ __device__ __forceinline__ void load_cell(const PT *__restrict__ P, const GridDe
   } else if (DIR == 2) {
     if (cs == 5) { jet_ambient(G, q); return; }  // reset to ambient, no y fill (conditions.f90:824-835)
     if (cs == 11) {  // reflecting poles, conditions.f90:977-988 (ny >= nghost enforced)
-      ld_cell(P, G, i, lo ? g : G.ny + 1 - g, k, q);
+      ld_cell<COHERENT>(P, G, i, lo ? g : G.ny + 1 - g, k, q);
       q[EQ_VY] = -q[EQ_VY];
       return;
     }
     if (cs == 12) {  // trans-polar, conditions.f90:1033-1050 (ny >= nghost, nz even enforced)
       int ks = k + G.nz / 2;
       if (ks > G.nz) ks -= G.nz;
-      ld_cell(P, G, i, lo ? g : G.ny + 1 - g, ks, q);
+      ld_cell<COHERENT>(P, G, i, lo ? g : G.ny + 1 - g, ks, q);
       q[EQ_VY] = -q[EQ_VY];
       return;
     }
-    ld_cell(P, G, i, wrap(j, G.ny), k, q);  // periodic
+    ld_cell<COHERENT>(P, G, i, wrap(j, G.ny), k, q);  // periodic
     return;
   } else {
     if (cs == 5) {  // nozzle inflow / reflecting wall below, outflow above, conditions.f90:851-869
@@ -298,16 +306,16 @@ __device__ __forceinline__ void load_cell(const PT *__restrict__ P, const GridDe
         if (G.xc[i + G.ng] <= G.jet[3]) {
           q[EQ_DE] = G.jet[4]; q[EQ_PR] = G.jet[5]; q[EQ_VX] = 0.0; q[EQ_VY] = 0.0; q[EQ_VZ] = G.jet[6];
         } else {
-          ld_cell(P, G, i, j, g, q);
+          ld_cell<COHERENT>(P, G, i, j, g, q);
           q[EQ_VZ] = -q[EQ_VZ];
         }
       } else {
-        ld_cell(P, G, i, j, G.nz, q);
+        ld_cell<COHERENT>(P, G, i, j, G.nz, q);
         q[EQ_VZ] = rmax(0.0, q[EQ_VZ]);
       }
       return;
     }
-    ld_cell(P, G, i, j, wrap(k, G.nz), q);  // periodic
+    ld_cell<COHERENT>(P, G, i, j, wrap(k, G.nz), q);  // periodic
   }
 }
 
