@@ -303,20 +303,29 @@ __device__ __forceinline__ void wavespeeds(const Phys &P, const R (&q)[NEQ], int
   wmin = rmin(rmin(rmin(R(0), e1), e2), e3);
 }
 
-// calc_hlle_fluxes, fluxes.f90:125-156; hlle_combine: one component from both sides
-template <class R>
-__device__ __forceinline__ R hlle_combine(R ap, R am, R fL, R fR, R uL, R uR) {
-  if (fabs(ap - am) < R(1.0e-14)) return R(0);
-  const R num = ap * fL - am * fR + ap * am * (uR - uL);
-  if (sizeof(R) == sizeof(float)) return num * (R(1) / (ap - am));  // as hlle: a reciprocal
-  return div_pos(num, ap - am);  // ap - am > 0 here (or NaN)
+// calc_hlle_fluxes, fluxes.f90:125-156.  hlle_combine: one component from both sides as
+// flux_and_cons_bare leaves them.  FP32 (the mixed policies): one reciprocal for the five
+// components, and every multiply-add spelled out, so that kernels which inline this in
+// different surroundings round alike (left to the compiler, the 1D stage kernel's two forms
+// contracted the difference of the conserved states differently, and a Michel flow's flux
+// differed at its sonic face, where ap is a rounding error).
+__device__ __forceinline__ float hlle_combine(float ap, float am, float inv, float sqg, float fL, float fR, float uL,
+                                              float uR) {
+  const float df = __fmaf_rn(ap, __fmul_rn(fL, sqg), -__fmul_rn(am, __fmul_rn(fR, sqg)));
+  const float du = __fmaf_rn(-uL, sqg, __fmul_rn(uR, sqg));
+  return __fmul_rn(__fmaf_rn(__fmul_rn(ap, am), du, df), inv);
+}
+__device__ __forceinline__ double hlle_combine(double ap, double am, double, double sqg, double fL, double fR, double uL,
+                                               double uR) {
+  fL = fL * sqg; fR = fR * sqg; uL = uL * sqg; uR = uR * sqg;
+  return div_pos(ap * fL - am * fR + ap * am * (uR - uL), ap - am);  // ap - am > 0 here (or NaN)
 }
 template <class R>
 __device__ __forceinline__ void hlle(const Phys &P, const R (&qL)[NEQ], const R (&qR)[NEQ], int dir,
                                      const FaceMetric<R> &m, R (&flux)[NEQ]) {
   R fL[NEQ], fR[NEQ], uL[NEQ], uR[NEQ], lLmin, lLmax, lRmin, lRmax;
-  flux_and_cons(P, qL, dir, m, fL, uL);
-  flux_and_cons(P, qR, dir, m, fR, uR);
+  flux_and_cons_bare(P, qL, dir, m, fL, uL);
+  flux_and_cons_bare(P, qR, dir, m, fR, uR);
   wavespeeds(P, qL, dir, m, lLmin, lLmax);
   wavespeeds(P, qR, dir, m, lRmin, lRmax);
   const R ap = rmax(rmax(R(0), lLmax), lRmax);
@@ -324,14 +333,10 @@ __device__ __forceinline__ void hlle(const Phys &P, const R (&qL)[NEQ], const R 
   if (fabs(ap - am) < R(1.0e-14)) {
 #pragma unroll
     for (int n = 0; n < NEQ; ++n) flux[n] = R(0);
-  } else if (sizeof(R) == sizeof(float)) {  // mixed policy: one reciprocal for the five components
-    const R inv = R(1) / (ap - am);
-#pragma unroll
-    for (int n = 0; n < NEQ; ++n) flux[n] = (ap * fL[n] - am * fR[n] + ap * am * (uR[n] - uL[n])) * inv;
   } else {
+    const R inv = sizeof(R) == sizeof(float) ? R(1) / (ap - am) : R(0);
 #pragma unroll
-    for (int n = 0; n < NEQ; ++n)  // ap - am > 0 here (or NaN)
-      flux[n] = div_pos(ap * fL[n] - am * fR[n] + ap * am * (uR[n] - uL[n]), ap - am);
+    for (int n = 0; n < NEQ; ++n) flux[n] = hlle_combine(ap, am, inv, m.sqg, fL[n], fR[n], uL[n], uR[n]);
   }
 }
 

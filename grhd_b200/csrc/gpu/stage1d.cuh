@@ -18,10 +18,12 @@
 //   4  (cell, variable): flux divergence, RK combination
 //   5  cell: con2prim
 // The expressions and their order are those of the other kernels, so FP64 results are the
-// same to the bit; in the mixed policy both states of a face are one thread's work, and the
-// HLLE sides stay without their sqrt(gamma) until they meet, so that the compiler contracts
-// the same multiply-add pairs as in the stage kernel: the FP32 fluxes of HLLE are the same to
-// the bit, con2prim's FP64 may differ in its last bits.  Measured: at STAGE1D_TILES_MAX in grhd2_gpu.cu.
+// same to the bit.  So are those of the mixed policies, whose multiply-add pairs the compiler
+// contracts: both states of a face are one thread's work and con2prim is the same inlined
+// function, whose pairs come out alike (their FP64 primitives compared before they are stored in
+// FP32: 409700 of 409700 equal, random states included); the HLLE combination and the RK stage
+// spell their pairs out.  (tests/test_gpu_stage1d_forms.py.)  Measured: at STAGE1D_TILES_MAX in
+// grhd2_gpu.cu.
 #pragma once
 
 #include "stage.cuh"
@@ -281,9 +283,12 @@ __global__ void __launch_bounds__(S1_BS, S1_MIN_BLOCKS)
         const R *l = s_fu + f, *r = s_fu + 12 * S1_FACES + f;
         const R ap = rmax(rmax(R(0), l[11 * S1_FACES]), r[11 * S1_FACES]);
         const R am = rmin(rmin(R(0), l[10 * S1_FACES]), r[10 * S1_FACES]);
-        const R fL = l[v * S1_FACES], fR = r[v * S1_FACES], uL = l[(NEQ + v) * S1_FACES], uR = r[(NEQ + v) * S1_FACES];
         const R sqg = s_t[FF_SQG * S1_FACES + f];
-        flux = hlle_combine(ap, am, fL * sqg, fR * sqg, uL * sqg, uR * sqg);
+        if (!(fabs(ap - am) < R(1.0e-14))) {
+          const R inv = sizeof(R) == sizeof(float) ? R(1) / (ap - am) : R(0);
+          flux = hlle_combine(ap, am, inv, sqg, l[v * S1_FACES], r[v * S1_FACES], l[(NEQ + v) * S1_FACES],
+                              r[(NEQ + v) * S1_FACES]);
+        }
       }
       s_f[v * S1_FACES + f] = flux;
     }
