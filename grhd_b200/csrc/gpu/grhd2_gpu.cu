@@ -404,17 +404,23 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
 }
 
 // The stage kernel's spread form (stage1d.cuh) runs 1D groups while all their tiles together
-// are resident at once: 148 SMs x 2 blocks of 63 cells.  It shortens a tile's dependent chain
-// but keeps most of a block's threads idle in its last phases, so beyond one wave the 256-cell
-// tiles win.  Measured per step, graph replays, 256-cell tiles and spread form: tubes of 400
-// cells (WENO5 + HLLE, 7 tiles each) FP64 1 grid 81 and 55 us, 32 grids 86 and 62, 128 grids
-// 108 and 171; MP5 + HLLC 117 and 87, 125 and 94, 158 and 265; Michel 1024 (17 tiles) 70 and 43,
-// 8 grids 71 and 44, 32 grids 72 and 84; mixed tube 39 and 25, Michel 39 and 25.  With the
-// launches overlapped (programmatic serialisation) and the clocks advanced in the last stage
-// the spread form's figures are 51 (tube FP64), 83 (HLLC), 41 (Michel), 19 and 21 us (mixed).
+// are resident at once: 148 SMs (a B200's) x 2 blocks of 63 cells.  It shortens a tile's
+// dependent chain but keeps most of a block's threads idle in its last phases, so beyond one wave
+// the 256-cell tiles win.  Measured per step, graph replays, 256-cell tiles and spread form:
+//   tubes of 400 cells (WENO5 + HLLE, 7 tiles each), FP64: 70 tiles 84 and 57 us, 287 86 and 59,
+//   350 86 and 76, 588 98 and 94; mixed 96 and 77, 98 and 79, 98 and 92, 105 and 104;
+//   MP5 + HLLC: 123 and 88, 126 and 91, 126 and 127, 141 and 167;
+//   Michel 1024 (17 tiles each): 68 tiles 70 and 40, 289 72 and 43, 340 71 and 78, 578 73 and 83;
+//   mixed 39 and 21, 39 and 23, 40 and 39, 41 and 41.
+// Several scheme groups share one batch's count (they run side by side): two to four groups of
+// 280 tiles together 93-131 and 63-100 us.  Batches on other streams are not counted.  Two at once
+// break even at the limit (287 tiles each: tubes 91 and 85, HLLC 133 and 134, Michel 73 and 73),
+// four do at half of it (140: 94 and 78, 133 and 122, 77 and 70); beyond, the spread form loses
+// what its idle threads cost (four of 287: 108 and 109, 159 and 217, 109 and 164), so 1D grids
+// belong in one batch.
 // Mixed HLLC groups keep the 256-cell tiles: in the spread form the compiler contracts other
-// multiply-add pairs of the FP32 HLLC, and its results would differ from the other kernels' by
-// 1e-7 on a tube (FP32 HLLE fluxes and reconstructions are the same to the bit).
+// multiply-add pairs of the FP32 HLLC, and a result would depend on the rest of its batch (1e-7 on
+// a tube).
 constexpr int STAGE1D_TILES_MAX = 148 * 2;
 
 // Whether a group's FP64 cell update runs in 256-thread blocks (cell.cuh): eight warps share
