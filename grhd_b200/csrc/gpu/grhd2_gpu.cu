@@ -1341,7 +1341,8 @@ static int copy_prims_in(grhd2_gpu *h, const double *p) {
 
 // The device's view of a state's host array when all of it is page-locked memory that kernels
 // can address, and it is small: the layout kernel then reads or writes it itself, without a
-// copy beside it.  NULL for other memory and larger arrays.  Measured, copy and direct: per
+// copy beside it.  NULL for other memory, larger arrays and addresses that are not a multiple of a
+// double's size, which a kernel cannot read and a copy engine can.  Measured, copy and direct: per
 // grid and call (8 grids in a loop) 15 KB 9.0 and 6.3 us, 80 KB 10.8 and 6.3, 160 KB 12.2 and
 // 10.3, 781 KB 26 and 22; 12 to 16 grids pipelined on four streams 80 KB 289 and 209 us, 121 KB
 // 238 and 221, but 252 KB 185 and 207, 781 KB 617 and 864: a larger array's PCIe time holds SMs
@@ -1349,7 +1350,7 @@ static int copy_prims_in(grhd2_gpu *h, const double *p) {
 constexpr size_t DIRECT_COPY_BYTES = (size_t)1 << 17;
 static double *device_view(const grhd2_gpu *h, const double *host) {
   const size_t bytes = h->n_interior * sizeof(double);
-  if (bytes > DIRECT_COPY_BYTES) return nullptr;
+  if (bytes > DIRECT_COPY_BYTES || (uintptr_t)host % sizeof(double) != 0) return nullptr;
   using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
   static const Query query = [] {
     void *f = nullptr;
