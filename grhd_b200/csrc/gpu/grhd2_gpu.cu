@@ -33,6 +33,7 @@
 #include "grhd2_gpu.h"
 #include "flux_launch.h"
 #include "frame.h"
+#include "prims_copy.h"
 #include "diag.cuh"
 #include "kernels.cuh"
 #include "metric_build.cuh"
@@ -1315,28 +1316,17 @@ int grhd2_gpu_set_bc_data(grhd2_gpu *h, const grhd2_gpu_bc_view *b) {
   return GRHD2_OK;
 }
 
-// The rows of the ghosted primitive array that k_prims_in reads, to the same places of the
-// staging buffer: the interior rows (with their ghosts along i, which rows j = 1..ny of a
-// plane hold contiguously) and, for two ghost cells, the rows at -nghost along the active
-// directions.  A 2D grid's ghost planes are most of its array: 27 MB against 3.4 MB of
-// interior rows for 400x1x200, 8.7 against 1.4 MB for 257x131x1.
+// The parts of the ghosted primitive array that k_prims_in reads (prims_copy.h), to the same
+// places of the staging buffer.
 static int copy_prims_in(grhd2_gpu *h, const double *p) {
   const grhd2_gpu_config &c = h->cfg;
-  const FortranLayout L{c.nx, c.ny, c.nz, c.nghost};
-  const size_t row = (size_t)5 * (c.nx + 2 * c.nghost + 1) * sizeof(double), plane = row * (c.ny + 2 * c.nghost + 1);
-  // rows j .. j + n - 1 of the planes k = 1..nz
-  auto rows = [&](int j, int n) {
-    const size_t off = (size_t)L.pidx(0, -c.nghost, j, 1);
-    if (c.nz == 1) return cudaMemcpyAsync(h->staging + off, p + off, n * row, cudaMemcpyHostToDevice, h->stream);
-    return cudaMemcpy2DAsync(h->staging + off, plane, p + off, plane, n * row, c.nz, cudaMemcpyHostToDevice, h->stream);
-  };
-  CUDA_TRY(h, rows(1, c.ny));
-  if (c.nghost == 2 && c.ny > 1) CUDA_TRY(h, rows(-c.nghost, 1));
-  if (c.nghost == 2 && c.nz > 1) {
-    const size_t off = (size_t)L.pidx(0, -c.nghost, 1, -c.nghost);
-    CUDA_TRY(h, cudaMemcpyAsync(h->staging + off, p + off, c.ny * row, cudaMemcpyHostToDevice, h->stream));
-  }
-  return GRHD2_OK;
+  return prims_in_pieces(c.nx, c.ny, c.nz, c.nghost, [&](const CopyPiece &x) -> int {
+    char *dst = (char *)h->staging + x.offset;
+    const char *src = (const char *)p + x.offset;
+    if (x.rows == 1) CUDA_TRY(h, cudaMemcpyAsync(dst, src, x.width, cudaMemcpyHostToDevice, h->stream));
+    else CUDA_TRY(h, cudaMemcpy2DAsync(dst, x.pitch, src, x.pitch, x.width, x.rows, cudaMemcpyHostToDevice, h->stream));
+    return GRHD2_OK;
+  });
 }
 
 // The device's view of a state's host array when all of it is page-locked memory that kernels
