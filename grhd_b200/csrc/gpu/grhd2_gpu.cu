@@ -1332,13 +1332,14 @@ static int copy_prims_in(grhd2_gpu *h, const double *p) {
 // The device's view of a state's host array when all of it is page-locked memory that kernels
 // can address, and it is small: the layout kernel then reads or writes it itself, without a
 // copy beside it.  NULL for other memory, larger arrays and addresses that are not a multiple of a
-// double's size, which a kernel cannot read and a copy engine can.  Measured, copy and direct: per
+// double's size, which a kernel cannot read and a copy engine can; and, where the kernel is to
+// write, for memory registered read-only.  Measured, copy and direct: per
 // grid and call (8 grids in a loop) 15 KB 9.0 and 6.3 us, 80 KB 10.8 and 6.3, 160 KB 12.2 and
 // 10.3, 781 KB 26 and 22; 12 to 16 grids pipelined on four streams 80 KB 289 and 209 us, 121 KB
 // 238 and 221, but 252 KB 185 and 207, 781 KB 617 and 864: a larger array's PCIe time holds SMs
 // that the other streams' steps want, so those keep the copy engines.
 constexpr size_t DIRECT_COPY_BYTES = (size_t)1 << 17;
-static double *device_view(const grhd2_gpu *h, const double *host) {
+static double *device_view(const grhd2_gpu *h, const double *host, bool write) {
   const size_t bytes = h->n_interior * sizeof(double);
   if (bytes > DIRECT_COPY_BYTES || (uintptr_t)host % sizeof(double) != 0) return nullptr;
   using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
@@ -1352,10 +1353,14 @@ static double *device_view(const grhd2_gpu *h, const double *host) {
   unsigned type = 0;
   CUdeviceptr dev = 0, start = 0;
   size_t size = 0;
-  CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
-                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-  void *out[4] = {&type, &dev, &start, &size};
-  if (query(4, what, out, (CUdeviceptr)host) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !dev) return nullptr;
+  unsigned long long access = 0;  // 1: read, 3: read and write
+  CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                 CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                 CU_POINTER_ATTRIBUTE_ACCESS_FLAGS};
+  void *out[5] = {&type, &dev, &start, &size, &access};
+  if (query(5, what, out, (CUdeviceptr)host) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !dev) return nullptr;
+  if (!(access & CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READ) || (write && access != CU_POINTER_ATTRIBUTE_ACCESS_FLAG_READWRITE))
+    return nullptr;
   const CUdeviceptr p = (CUdeviceptr)host;  // all of the array inside the locked range
   return p >= start && p - start <= size && size - (p - start) >= bytes ? (double *)dev : nullptr;
 }
@@ -1376,7 +1381,7 @@ static int upload_impl(grhd2_gpu *h, const double *up, const double *p, bool syn
     h->prims_set = true;
   }
   if (up) {
-    const double *src = device_view(h, up);
+    const double *src = device_view(h, up, false);
     if (!src) {
       CUDA_TRY(h, cudaMemcpyAsync(h->staging, up, h->n_interior * sizeof(double), cudaMemcpyHostToDevice, h->stream));
       src = h->staging;
@@ -1532,7 +1537,7 @@ static int download_impl(grhd2_gpu *h, double *up, double *p, bool sync) {
   }
   if (up) {
     if (!h->cons_set) return fail(h, GRHD2_ERR_STATE, "conserved state not uploaded");
-    double *dst = device_view(h, up);
+    double *dst = device_view(h, up, true);
     k_cons_out<<<nblocks(G.ncell, LAYOUT_BS), LAYOUT_BS, 0, h->stream>>>(G, G.UP, dst ? dst : h->staging);
     if (int rc = launch_check(h)) return rc;
     if (!dst)
