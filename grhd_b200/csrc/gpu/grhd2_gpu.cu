@@ -355,17 +355,22 @@ TuneKey tune_key(const Group &grp, const std::vector<GridDev> &hg, int dir) {
 // direction.  Measured per step on batches of 1 to 32 tori 400x1x200 (80k faces each), 3D
 // tori of 48x24x24 to 256x128x128 and x-z grids of 256x128, us for split, split per variable
 // and fused:
-//   mixed: fused throughout (70 against 77-83 at 33k faces; tori 106 against 118-124 at 80k,
-//     1512 against 1910 at 2.6M; 3D torus MP5 + HLLC 3536 against 4267)
+//   mixed: fused (70 against 77-83 at 33k faces; tori 106 against 118-124 at 80k, 1512 against
+//     1910 at 2.6M; 3D torus MP5 + HLLC 3536 against 4267; x-y grids 85 against 89 split per
+//     variable at 2k and 85-95 against 91-101 at 8k; 3D grids level at 1k and 8k, 115 against 122
+//     at 16k), but x-z grids below about 8k faces split per variable, whose items per face are
+//     shorter (HLLE 62 against 66 and HLLC 75 against 79 at 2.3k, 80.4 and 82.3, 91 and 95 at 4k,
+//     80.5 and 82.1, 88 and 92 at 5.4k; at 8k 76.0 and 75.8, 84.6 and 84.2, at 13k 77.4 and 74.1).
+//     The variants agree to the bit, so the choice shows in no result (test_gpu_mixed_variants.py)
 //   FP64 HLLE: fused from 80k faces (167 against 189 and 181; 3006 against 3251 and 3614 at
 //     2.6M), split per variable at 33k (117 against 142 and 130) and 28k (186, 220, 190), whose
 //     one thread per face would leave SMs idle
 //   FP64 HLLC, whose fused form spills: split from 160k faces (356 against 397 and 364; 3D
 //     torus 8183 against 11315 and 9772), at 80k level (241, 237, 244), split per variable below
 //     (288, 253, 252 at 28k)
-constexpr long long FUSED_FROM_FACES = 60000, SPLIT_FROM_FACES = 120000;
-int default_variant(bool mixed, int rs, long long faces) {
-  if (mixed) return GRHD2_FLUX_FUSED;
+constexpr long long FUSED_FROM_FACES = 60000, SPLIT_FROM_FACES = 120000, MIXED_XZ_FUSED_FROM_FACES = 8000;
+int default_variant(bool mixed, int rs, int sd, long long faces) {
+  if (mixed) return sd == 3 && faces < MIXED_XZ_FUSED_FROM_FACES ? GRHD2_FLUX_SPLIT_VAR : GRHD2_FLUX_FUSED;
   if (rs == RS_HLLE) return faces >= FUSED_FROM_FACES ? GRHD2_FLUX_FUSED : GRHD2_FLUX_SPLIT_VAR;
   return faces >= SPLIT_FROM_FACES ? GRHD2_FLUX_SPLIT : GRHD2_FLUX_SPLIT_VAR;
 }
@@ -380,7 +385,7 @@ FluxChoice choose_flux(const grhd2_gpu_batch *b, int gi, const Group &grp, const
   if (f != b->forced.end()) return f->second;
   long long faces = 0;
   for (int g : grp.members) faces += face_count(hg[g], dir);
-  FluxChoice c{default_variant(grp.mixed, grp.rs, faces), DEFAULT_TX};
+  FluxChoice c{default_variant(grp.mixed, grp.rs, grp.sd, faces), DEFAULT_TX};
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune.find(tune_key(grp, hg, dir));

@@ -304,8 +304,8 @@ int grhd2_gpu_batch_profile_step(grhd2_gpu_batch *b, float *ms, const char **nam
 int grhd2_gpu_batch_clocks(grhd2_gpu_batch *b, double *t, int64_t *steps, int *active);
 /* Kernel variants of the face fluxes of one direction. */
 #define GRHD2_FLUX_AUTO -1      /* the autotuned choice for this shape if one is cached, else FUSED for the mixed
-                                   policies and for FP64 HLLE launches from 60k faces, SPLIT for FP64 HLLC
-                                   from 120k, SPLIT_VAR below */
+                                   policies (x-z grids: from 8k faces) and for FP64 HLLE launches from 60k
+                                   faces, SPLIT for FP64 HLLC from 120k, SPLIT_VAR below */
 #define GRHD2_FLUX_SPLIT 0      /* reconstruction kernel (thread per face) + Riemann kernel */
 #define GRHD2_FLUX_FUSED 1      /* one kernel, thread per face, interface states kept on chip */
 #define GRHD2_FLUX_SPLIT_VAR 2  /* reconstruction kernel (thread per face and variable) + Riemann kernel */
