@@ -519,17 +519,26 @@ int build_batch(grhd2_gpu_batch *b) {
   BCUDA_TRY(b, cudaMallocAsync((void **)&b->d_grids, sizeof(GridDev) * n, b->stream));
   BCUDA_TRY(b, cudaMallocAsync((void **)&b->d_clocks, sizeof(GridClock) * n, b->stream));
   BCUDA_TRY(b, cudaMemcpyAsync(b->d_grids, hg.data(), sizeof(GridDev) * n, cudaMemcpyHostToDevice, b->stream));
+  // blocks of every kernel kind, and the forms they decide
+  int tiles1d = 0;  // the groups of a step run side by side: their tiles share the GPU
   for (auto &grp : b->groups) {
+    for (int k = 0; k < NKIND; ++k)
+      for (int g : grp.members) grp.nb[k] += (int)((kind_items(hg[g], k) + KIND_BS[k] - 1) / KIND_BS[k]);
+    grp.cell_wide = use_wide_cells(grp, hg);
+    if (grp.stage && grp.sd == 0) tiles1d += grp.nb[K_STAGE1D];
+  }
+  for (auto &grp : b->groups) {
+    grp.stage1d = grp.stage && grp.sd == 0 && tiles1d <= STAGE1D_TILES_MAX && !(grp.mixed && grp.rs == RS_HLLC);
+    if (!grp.cell_wide) grp.nb[K_CELL_WIDE] = 0;  // no map for a form the group does not take
+    if (!grp.stage1d) grp.nb[K_STAGE1D] = 0;
     std::vector<BlockMap> map;
     for (int k = 0; k < NKIND; ++k) {
       grp.off[k] = (int)map.size();
       for (int g : grp.members) {
-        const long long items = kind_items(hg[g], k);
+        const long long items = grp.nb[k] > 0 ? kind_items(hg[g], k) : 0;
         for (long long first = 0; first < items; first += KIND_BS[k]) map.push_back(BlockMap{g, (int)first});
       }
-      grp.nb[k] = (int)map.size() - grp.off[k];
     }
-    grp.cell_wide = use_wide_cells(grp, hg);
     BCUDA_TRY(b, cudaMallocAsync((void **)&grp.d_map, sizeof(BlockMap) * std::max<size_t>(1, map.size()), b->stream));
     BCUDA_TRY(b, cudaMemcpyAsync(grp.d_map, map.data(), sizeof(BlockMap) * map.size(), cudaMemcpyHostToDevice, b->stream));
     // persistent kernel: flattened item spaces (faces of every active direction; cells)
@@ -565,11 +574,7 @@ int build_batch(grhd2_gpu_batch *b) {
       if (e != cudaSuccess) return bfail(b, GRHD2_ERR_CUDA, "persistent stage kernel occupancy: %s", cudaGetErrorString(e));
     }
   }
-  int tiles1d = 0;  // the groups of a step run side by side: their tiles share the GPU
-  for (const auto &grp : b->groups)
-    if (grp.stage && grp.sd == 0) tiles1d += grp.nb[K_STAGE1D];
   for (auto &grp : b->groups) {
-    grp.stage1d = grp.stage && grp.sd == 0 && tiles1d <= STAGE1D_TILES_MAX && !(grp.mixed && grp.rs == RS_HLLC);
     if (!grp.stage1d) continue;
     cudaError_t e = grp.mixed ? stage1d_setup<float, float>(grp.rec, grp.rs) : stage1d_setup<double, double>(grp.rec, grp.rs);
     if (e != cudaSuccess) return bfail(b, GRHD2_ERR_CUDA, "1D stage kernel set-up: %s", cudaGetErrorString(e));
