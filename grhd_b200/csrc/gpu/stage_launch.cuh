@@ -42,9 +42,12 @@ void launch_stage_sd(int rec, int rs, int mode, const GridDev *grids, const Bloc
 
 // the spread form for small launches of 1D grids (stage1d.cuh)
 static_assert(S1_BS == STAGE1D_BLOCK && S1_CELLS == STAGE1D_CELLS, "the host's tile geometry is the kernel's");
+// (mixed HLLC groups never take it: STAGE1D_TILES_MAX in grhd2_gpu.cu)
 template <int REC, class R, class PT>
 inline const void *stage1d_fn(int rs) {
-  return rs == RS_HLLC ? (const void *)k_stage1d<REC, RS_HLLC, R, PT> : (const void *)k_stage1d<REC, RS_HLLE, R, PT>;
+  if constexpr (sizeof(R) == sizeof(double))
+    if (rs == RS_HLLC) return (const void *)k_stage1d<REC, RS_HLLC, R, PT>;
+  return rs == RS_HLLE ? (const void *)k_stage1d<REC, RS_HLLE, R, PT> : nullptr;
 }
 template <class R, class PT>
 inline const void *stage1d_kernel(int rec, int rs) {
