@@ -692,8 +692,14 @@ __device__ inline double root_brent(double g1, double rho_floor, double D, doubl
 }
 // FP32 estimate of the residual and its derivative for E = tau + D scaled out:
 // f / E^2 and f' / E^2 at W, d = D / E, q = Q2 / E^2.  For g1 >= 1.9 and |d| <= 1.25 the term
-// V^2 (1 - 1/W^2) is at most 2 and V^2 at most 12, so the error of f is below 1.1e-5 (about 90
-// roundings of terms of order one) and that of f' below 1e-5 (1 + |d| W) / W^3.
+// V^2 (1 - 1/W^2) is at most 2 and V^2 at most 12.25 (W = 1, d = -1.25).  The errors, emulated in
+// FP32 with exact division over 3.2e7 operands of that domain, W from 1 + 1e-8 to 1e5, q to 2, and
+// with the rounding of W: 2.7e-6 of f and 1.6e-5 (1 + |d| W) / W^3 of f'; the approximate
+// divisions (2 ulp) take them to no more than 1.1e-5 and 3e-5.  A bisection's decision compares
+// 2 |f| with |dx_old f'|, where dx_old <= 4 (W - 1): 4 (W - 1) (1 + 1.25 W) / W^3 is at most 1.8,
+// so its margin of 1e-4 exceeds 2.2e-5 + 1.8 * 3e-5.  q is not bounded: for large q the sign of
+// f is certain (the other term is at most 2), and its error of 3 roundings, 2e-7 q, is far below
+// the comparison's relative slack of 1 %.
 struct RootScreen {
   float g1, d, q;
   __device__ __forceinline__ void eval(float W, float &f, float &df) const {
