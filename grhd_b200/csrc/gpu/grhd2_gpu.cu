@@ -430,8 +430,10 @@ bool use_stage(const grhd2_gpu_batch *b, const Group &grp) {
 constexpr int STAGE1D_TILES_MAX = 148 * 2;
 
 // Whether a group's FP64 cell update runs in 256-thread blocks (cell.cuh): eight warps share
-// a table slice instead of four, which leaves L1 75 KB more and shared memory room to stage
-// up and u.  Measured on k tori of 400x1x200 (325 wide blocks each), us per stage, narrow and
+// a table slice instead of four, and the 76 KB per SM that saves pay for staging up and u (82 KB;
+// L1 keeps what it had).  The staging is most of the gain: half batch of the 32 tori and 3D torus,
+// us per stage, 128 threads 195 and 580, 256 threads without staging 192 and 580, with it 183
+// and 550.  Measured on k tori of 400x1x200 (325 wide blocks each), us per stage, narrow and
 // wide: k = 1 25.2 and 27.4, k = 2 38.0 and 36.2, k = 4 62.8 and 59.1, k = 12 157 and 146,
 // k = 32 405 and 376; 3D torus 256x128x128 635 and 568.  So wide blocks pay once they fill the
 // GPU (148 SMs x 4 resident blocks) more than once; below that the coarser blocks leave SMs
