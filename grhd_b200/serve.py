@@ -11,7 +11,7 @@ transfer, retires finished grids (result downloaded, memory released) and rebuil
 batch if its membership changed.  State never leaves the device between steps.
 
 The reference runs such sweeps as independent processes (one Fortran run per problem,
-``inundaciones.sh``); a grid's result here is the result it has alone (FP64: bitwise).
+``inundaciones.sh``); a grid's result here is the result it has alone, bit for bit.
 
     python -m grhd_b200.serve --requests 4096 --rate 2000 --michel-final-time 50
 """
